@@ -89,4 +89,19 @@ __device__ __forceinline__ void bulk_copy_g2s(void* smem, const void* gmem, unsi
         : "memory");
 }
 
+// Bulk copy of `bytes` (multiple of 16; both addresses 16-byte aligned) from
+// this CTA's shared memory to global, as a bulk group of the calling thread.
+__device__ __forceinline__ void bulk_copy_s2g(void* gmem, const void* smem, unsigned bytes) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile(
+        "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n"
+        "cp.async.bulk.commit_group;\n" ::"l"(gmem),
+        "r"(s), "r"(bytes)
+        : "memory");
+}
+
+// Wait until the calling thread's bulk stores have read their source / are complete.
+__device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_wait() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+
 }  // namespace gmpm

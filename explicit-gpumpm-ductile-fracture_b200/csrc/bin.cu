@@ -395,7 +395,7 @@ void batch_scene_ctas(int64_t n, uint32_t key_space, int nb_cap, int ng_cap, int
     ctas[BM_ZERO_CELLS] = cdiv(ncell * 4, 4096);
     ctas[BM_CELL_TILES] = cdiv(ncell, kScanTile);
     ctas[BM_CANON] = std::max(1, std::min(cdiv(nb_cap, kCanonWarps), sms * 8));
-    ctas[BM_P2G] = std::max(1, std::min(nb_cap, sms));
+    ctas[BM_P2G] = real_bytes == 4 ? p2g_ctas<float>(nb_cap, sms) : p2g_ctas<double>(nb_cap, sms);
     ctas[BM_GRID] = std::max(1, std::min(ng_cap / 4 + 1, sms * 8));
     const int per_sm = real_bytes == 4 ? 2 : 1;  // G2P's resident CTAs per SM
     ctas[BM_G2P] = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * per_sm));

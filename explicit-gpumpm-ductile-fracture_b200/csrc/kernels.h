@@ -86,6 +86,10 @@ template <typename R>
 cudaError_t launch_p2g(const SceneDev<R>* sc, const PState<R>& st, const PAux<R>& aux, BinDev bin, GridDev grid,
                        Counters* cnt, LaunchCfg cfg, cudaStream_t stream);
 
+// CTAs of a one-scene P2G launch sized for `sms` SMs.
+template <typename R>
+int p2g_ctas(int nb_cap, int sms);
+
 template <typename R>
 cudaError_t launch_grid(const SceneDev<R>* sc, BinDev bin, GridDev grid, Counters* cnt, LaunchCfg cfg,
                         cudaStream_t stream);

@@ -2,35 +2,46 @@
 // P2GKernal.cu:512-702) plus the phase-field channels (volP2G_APIC,
 // preConditionP2G_APIC, AxP2G_APIC: P2GKernal.cu:897-1326).
 //
-// Each CTA walks its particle pages (grid-stride) in chunks of up to
-// P2GChunk sorted slots (a whole page of 8 particles per cell in FP32).  A
-// page's particles share the page's 6x6x6 node window and, within a cell,
-// the same 3x3x3 stencil.  Between substeps the particle planes are in the
-// previous sorted order and perm is close to the identity, so the 28 raw
-// input planes of the next chunk are fetched as contiguous windows of
-// previous slots with bulk copies (one thread issues them; the tensor memory
-// accelerator moves the data) while the current chunk is swept.  Particles
-// whose previous slot falls outside the window (they changed page) are read
-// directly.  Each thread then turns one particle's raw words into a 44-word
-// record.
+// Each CTA walks its particle pages (grid-stride) in chunks of up to kP2GChunk
+// sorted slots (a whole page of 8 particles per cell).  A page's particles
+// share the page's 6x6x6 node window and, within a cell, the same 3x3x3
+// stencil.  Between substeps the particle planes are in the previous sorted
+// order and perm is close to the identity, so the 28 raw input planes of a
+// chunk are fetched as contiguous windows of previous slots with bulk copies
+// (one thread issues them; the tensor memory accelerator moves the data) and
+// read where they land, through the slot's place in the window.  A chunk with
+// a particle whose previous slot falls outside the window (it changed page) is
+// first gathered into sorted order in shared memory.
 //
-// Work split: one warp per cell z-column (cx, cy) of the page; lane
-// (g, i, j) = channel group g (0..2) x stencil column (i, j).  A warp sweeps
-// its column's cells (cx, cy, 0..3) in order, all lanes on the same particle,
-// so control flow is uniform.  Lane (g, i, j) owns window nodes
-// (cx+i, cy+j, 0..5) for its group's three channels:
-//   g = 0: momentum x, mass, damage weight
-//   g = 1: momentum y, weight, V w
-//   g = 2: momentum z, V w FP, grad w . q (phase-field flux)
-// Every particle of cell cz adds to nodes cz..cz+2 with register indices
-// fixed at compile time (the sweep over cz is unrolled), so the sums stay in
-// registers: no shuffles and no per-particle atomics.
+// Work split: one lane per cell and channel group.  A lane walks its cell's
+// particles and keeps the cell's 27 node sums of its channels in registers, so
+// a particle costs each lane its weights once and 27 fused multiply-adds per
+// term and channel, with no shuffles and no atomics.  The groups, one per pair
+// of warps, hold two channels per packed FP32 instruction (fma.rn.f32x2):
+//   0: momentum x, y        1: momentum z, grad w . q
+//   2: mass, damage weight  3: weight, V w, V w FP
+// With w = X_i Y_j Z_k, the momentum of node (i, j, k) is
+//   P_i (Y_j Z_k) + X_i (Y_j U_k + Q_j Z_k),
+// where P, Q and U hold the APIC and stress terms of one axis each:
+//   P_i = b_x (i - d_x) X_i + s_x X'_i, Q likewise, U_k with the velocity term.
+// Lane l of a group's first warp takes the fuller of cells l and l + 32, and of
+// its second warp the other, so that a warp's lanes hold cells of similar
+// counts (its loop runs as long as its fullest cell).
 //
-// Deterministic mode: after a page's last chunk the column sums are gathered
-// per window node in a fixed order (at most 9 terms, compensated) and written once to the
-// page's tile in HBM, so results are bitwise reproducible.  Fast mode:
-// columns add into a shared tile with atomics.  The grid kernel sums the
-// eight page tiles overlapping each grid page in fixed slot order either way.
+// The page's cell sums then go to shared memory (over the staged planes) and
+// are gathered per window node in a fixed order (gather_item) into the page's
+// tile, which one bulk copy writes to HBM.  Results are bitwise reproducible
+// in both modes of the scene.  The grid kernel sums the eight page tiles
+// overlapping each grid page in fixed slot order.
+//
+// Bound: neither HBM (17% of the copy rate) nor one pipe, but the chain of a
+// page's phases (copy 2,000 cycles, sweep 9,000, gather 3,000), which the two
+// CTAs of an SM overlap in part: 54% of the issue slots, FMA pipe 46%, shared
+// memory 49%.  Measured on FP32 plates: 0.718 ms at 8.4M particles and 2.73 ms
+// at 33.5M, where one lane per stencil column, all lanes on the same particle,
+// took 1.209 and 4.67 (88 warp instructions a particle against 51: every
+// particle's words were read, and its weights formed, by 27 lanes).  FP64 at
+// 1.1M particles: 0.245 against 0.391 ms.
 #include <cstdint>
 
 #include "async_copy.cuh"
@@ -39,48 +50,16 @@
 
 namespace gmpm {
 
-constexpr int kP2GWarps = 16;  // one per cell z-column (cx, cy)
-constexpr int kP2GThreads = 32 * kP2GWarps;
-constexpr int kColumns = 144;  // 16 cell z-columns x 9 stencil columns
-// Page flush: column sums channel-major, [channel][stencil column (144)][z (6)], the channel stride padded
-// so that the three channel groups of a warp's stores fall in different banks.  A gather step of one
-// channel over consecutive window nodes then reads consecutive words.
-constexpr int kFlushChStride = kColumns * 6 + 8;
-constexpr int kRec = 44;       // words per staged particle record
-
-template <typename R> struct P2GChunk;
-template <> struct P2GChunk<float> { static constexpr int value = 512; };
-template <> struct P2GChunk<double> { static constexpr int value = 256; };
-
-// Record layout: 8 common words (the x and y offsets from the base node in
-// cells, xp/dx; the three z weights and their gradients), then one 12-word
-// block per channel group g at RF_BLOCK + 12 g:
-//   U, A0, A1, A2 | S0, S1, S2, s1 | t0, t1, t2, t3
-// with, for a lane of stencil column (i, j) and node k of the sweep,
-//   momentum_g += w (U + A0 i + A1 j + A2 k) + (S0 gxy0 + S1 gxy1) wz + S2 wxy gz
-//   second     += s1 w
-//   third      += (t0 wxy + t1 gxy0 + t2 gxy1) wz + t3 wxy gz
-// where U = m v_g - (m B D^-1 xp)_g, A = dx (m B D^-1) row g, S = -dt V0 P F^T
-// row g.  s1 = (m, 1, V FP); t = (c,0,0,0), (V,0,0,0), (0, q0, q1, q2).
-enum RecField : int { RF_XP0 = 0, RF_XP1 = 1, RF_WZ = 2, RF_GZ = 5, RF_BLOCK = 8 };
-static_assert(RF_BLOCK + 3 * 12 == kRec, "record layout");
+constexpr int kP2GGroups = 4;
+constexpr int kP2GThreads = 64 * kP2GGroups;  // two warps (64 cells) per channel group
+constexpr int kP2GChunk = 576;
+template <typename R>
+constexpr int p2g_ctas_per_sm() { return sizeof(R) == 4 ? 2 : 1; }  // by registers and shared memory
 
 // Raw particle planes, in staging order.
 enum RawField : int {
     RW_X = 0, RW_V = 3, RW_B = 6, RW_SIG = 15, RW_C = 21, RW_M = 22, RW_VOL = 23, RW_FP = 24, RW_Q = 25,
     kRawWords = 28
-};
-
-// Staging window of previous slots: the chunk's CH slots plus kMargin on
-// either side; planes padded in shared memory to spread banks.
-constexpr int kMargin = 64;
-template <typename R>
-struct Staging {
-    static constexpr int CH = P2GChunk<R>::value;
-    static constexpr int W = CH + 2 * kMargin;             // window length (elements)
-    static constexpr int WS = W + (int)(16 / sizeof(R));   // plane stride in shared memory
-    static_assert(W <= kPlanePad, "window fits the plane padding");
-    static_assert((W * sizeof(R)) % 16 == 0 && (WS * sizeof(R)) % 16 == 0, "bulk copy granularity");
 };
 
 // Device pointer of raw plane q.
@@ -97,155 +76,219 @@ __device__ __forceinline__ const R* raw_plane(const PState<R>& st, const PAux<R>
     return aux.q[q - RW_Q];
 }
 
+// Staging window of previous slots: the chunk's slots plus kMargin on either
+// side; planes padded in shared memory to spread banks.
+constexpr int kMargin = 64;
 template <typename R>
-__device__ __forceinline__ void bspline1d(R xp, R inv_dx, R* w, R* g) {
-    // quadratic B-spline weights and gradients on nodes base+0..2, xp relative
-    // to the base node (P2GKernal.cu:590-611)
-    R d0 = xp * inv_dx;
-    R z = R(1.5) - d0;
-    w[0] = R(0.5) * z * z;
-    g[0] = -z * inv_dx;
-    d0 = d0 - R(1);
-    w[1] = R(0.75) - d0 * d0;
-    g[1] = -d0 * R(2) * inv_dx;
-    z = R(1.5) - (R(1) - d0);
-    w[2] = R(0.5) * z * z;
-    g[2] = z * inv_dx;
+struct Staging {
+    static constexpr int W = kP2GChunk + 2 * kMargin;      // longest window (elements)
+    static constexpr int WS = W + (int)(16 / sizeof(R));   // plane stride in shared memory
+    static_assert(W <= kPlanePad, "window fits the plane padding");
+    static_assert((W * sizeof(R)) % 16 == 0 && (WS * sizeof(R)) % 16 == 0, "bulk copy granularity");
+};
+__device__ __forceinline__ int window_length(int n) { return (n + 2 * kMargin + 3) & ~3; }
+
+// Two channels of one value.  FP32: Blackwell's packed instructions.
+template <typename R> struct Pk;
+template <> struct Pk<float> { using T = float2; };
+template <> struct Pk<double> { using T = double2; };
+template <typename R> using pk_t = typename Pk<R>::T;
+__device__ __forceinline__ float2 pk(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 pk(double a, double b) { return make_double2(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
+    return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+template <typename R>
+__device__ __forceinline__ pk_t<R> dup(R a) { return pk(a, a); }
+
+// quadratic B-spline weights on nodes base+0..2 and their gradients times dx,
+// d = (x - x_base) / dx (P2GKernal.cu:590-611)
+template <typename R>
+__device__ __forceinline__ void bspline1d(R d, R* w, R* h) {
+    const R z0 = R(1.5) - d, z1 = d - R(1), z2 = d - R(0.5);
+    w[0] = R(0.5) * z0 * z0;
+    w[1] = R(0.75) - z1 * z1;
+    w[2] = R(0.5) * z2 * z2;
+    h[0] = -z0;
+    h[1] = R(-2) * z1;
+    h[2] = z2;
 }
 
-// Build the particle's record from its raw words.
-template <typename R>
-__device__ __forceinline__ void build_record(const SceneDev<R>* __restrict__ sc, const int base[3], const R* raw,
-                                             R* rec) {
-    const R dx = sc->dx, inv_dx = sc->inv_dx, dt = sc->dt, Dinv = sc->Dinv;
-    R xp[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) xp[a] = raw[RW_X + a] - R(base[a]) * dx;
-    R out[kRec];
-    // x and y offsets in cells: the product every lane's weight needs, formed once
-    out[RF_XP0] = xp[0] * inv_dx;
-    out[RF_XP1] = xp[1] * inv_dx;
-    bspline1d(xp[2], inv_dx, out + RF_WZ, out + RF_GZ);
-    const R m = raw[RW_M];
-    const R V = raw[RW_VOL];
-    R mB[9];  // m B D^-1, (r,c) at 3r+c; B planes are column-major (r + 3c)
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) mB[3 * r + c] = m * raw[RW_B + r + 3 * c] * Dinv;
-    // -dt sigma, sigma stored xx yy zz xy xz yz
-    R S[9];
-    S[0] = -dt * raw[RW_SIG + 0];
-    S[4] = -dt * raw[RW_SIG + 1];
-    S[8] = -dt * raw[RW_SIG + 2];
-    S[1] = S[3] = -dt * raw[RW_SIG + 3];
-    S[2] = S[6] = -dt * raw[RW_SIG + 4];
-    S[5] = S[7] = -dt * raw[RW_SIG + 5];
-#pragma unroll
-    for (int g = 0; g < 3; ++g) {
-        R* blk = out + RF_BLOCK + 12 * g;
-        blk[0] = m * raw[RW_V + g] - (mB[3 * g] * xp[0] + mB[3 * g + 1] * xp[1] + mB[3 * g + 2] * xp[2]);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            blk[1 + c] = dx * mB[3 * g + c];
-            blk[4 + c] = S[3 * g + c];
-        }
-    }
-    R* b0 = out + RF_BLOCK;
-    R* b1 = b0 + 12;
-    R* b2 = b1 + 12;
-    b0[7] = m;
-    b0[8] = raw[RW_C];
-    b0[9] = b0[10] = b0[11] = R(0);
-    b1[7] = R(1);
-    b1[8] = V;
-    b1[9] = b1[10] = b1[11] = R(0);
-    b2[7] = V * raw[RW_FP];
-    b2[8] = R(0);
-    b2[9] = raw[RW_Q + 0];
-    b2[10] = raw[RW_Q + 1];
-    b2[11] = raw[RW_Q + 2];
-    static_assert((kRec * sizeof(R)) % 16 == 0, "record must be whole 16-byte words");
-#pragma unroll
-    for (int q = 0; q < (int)(kRec * sizeof(R) / 16); ++q)
-        reinterpret_cast<uint4*>(rec)[q] = reinterpret_cast<const uint4*>(out)[q];
+template <typename P>
+__device__ __forceinline__ void kahan_add2(P& s, P& c, P v) {
+    const P minus = pk(decltype(s.x)(-1), decltype(s.x)(-1));
+    const P y = fma2(c, minus, v);
+    const P t = add2(s, y);
+    c = fma2(y, minus, fma2(s, minus, t));
+    s = t;
+}
+// The CTA's barrier at points where warps of different groups arrive from
+// different code (barrier 1; __syncthreads uses barrier 0).
+__device__ __forceinline__ void p2g_barrier() {
+    asm volatile("bar.sync 1, %0;\n" ::"n"(kP2GThreads) : "memory");
 }
 
-// Per-lane constants of the B-spline piece of stencil node i along one axis,
-// written around z = xp/dx - shift: w = a z^2 + b, dw/dx = c z.
+// What a lane keeps about its cell and the scene.
 template <typename R>
-struct Piece {
-    R shift, a, b, c;
-    __device__ __forceinline__ void init(int i, R inv_dx) {
-        shift = i == 0 ? R(1.5) : (i == 1 ? R(1) : R(0.5));
-        a = i == 1 ? R(-1) : R(0.5);
-        b = i == 1 ? R(0.75) : R(0);
-        c = (i == 1 ? R(-2) : R(1)) * inv_dx;
-    }
-    __device__ __forceinline__ void eval(R xp_over_dx, R& w, R& g) const {
-        const R z = xp_over_dx - shift;
-        w = a * (z * z) + b;
-        g = c * z;
-    }
+struct LaneCell {
+    R b[3];           // base node coordinates
+    R dx, inv_dx, kD, kS;  // kD = dx D^-1, kS = -dt / dx
 };
 
-template <int NW, typename R>
-__device__ __forceinline__ void load_words(const R* __restrict__ src, R* dst) {
-    static_assert((NW * sizeof(R)) % 16 == 0, "whole 16-byte words");
-#pragma unroll
-    for (int q = 0; q < (int)(NW * sizeof(R) / 16); ++q)
-        reinterpret_cast<uint4*>(dst)[q] = reinterpret_cast<const uint4*>(src)[q];
-}
+// Staged words of a group's particle, x y z first.
+__device__ constexpr int kWordsXY[17] = {RW_X,     RW_X + 1, RW_X + 2, RW_M,       RW_V,       RW_V + 1,
+                                         RW_B,     RW_B + 1, RW_B + 3, RW_B + 4,   RW_B + 6,   RW_B + 7,
+                                         RW_SIG,   RW_SIG + 1, RW_SIG + 3, RW_SIG + 4, RW_SIG + 5};
+__device__ constexpr int kWordsZQ[14] = {RW_X,     RW_X + 1, RW_X + 2,   RW_M,       RW_V + 2,   RW_B + 2, RW_B + 5,
+                                         RW_B + 8, RW_SIG + 4, RW_SIG + 5, RW_SIG + 2, RW_Q,     RW_Q + 1, RW_Q + 2};
+__device__ constexpr int kWordsMC[5] = {RW_X, RW_X + 1, RW_X + 2, RW_M, RW_C};
+__device__ constexpr int kWordsV[5] = {RW_X, RW_X + 1, RW_X + 2, RW_VOL, RW_FP};
 
-// One particle of cell z-index CZ into a lane's 6 z-nodes x 3 channels.
-template <int CZ, typename R>
-__device__ __forceinline__ void accumulate(const R* __restrict__ rec, int g, const Piece<R>& px, const Piece<R>& py,
-                                           R fi, R fj, R* acc) {
-    R cw[8], bw[12];
-    load_words<8>(rec, cw);
-    load_words<12>(rec + RF_BLOCK + 12 * g, bw);
-    R wx, gx, wy, gy;
-    px.eval(cw[RF_XP0], wx, gx);
-    py.eval(cw[RF_XP1], wy, gy);
-    const R wxy = wx * wy, gxy0 = gx * wy, gxy1 = wx * gy;
-    const R al = bw[4] * gxy0 + bw[5] * gxy1, be = bw[6] * wxy;
-    const R s1w = bw[7] * wxy;
-    const R gam = bw[8] * wxy + bw[9] * gxy0 + bw[10] * gxy1, del = bw[11] * wxy;
-    // momentum at node k: wz (wxy u_k + al) + gz be with u_k = u0 + k A2, i.e.
-    // wz (alpha + k beta) + gz be
-    const R u0 = bw[0] + bw[1] * fi + bw[2] * fj;
-    const R alpha = wxy * u0 + al, beta = wxy * bw[3];
+template <typename R>
+__device__ __forceinline__ void particle_weights(const R* x, const LaneCell<R>& L, R d[3], R w[3][3], R h[3][3]) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const R wz = cw[RF_WZ + k], gz = cw[RF_GZ + k];
-        const R tk = k == 0 ? alpha : (k == 1 ? alpha + beta : alpha + R(2) * beta);
-        R* A = acc + 3 * (CZ + k);
-        A[0] += wz * tk + be * gz;
-        A[1] += s1w * wz;
-        A[2] += gam * wz + del * gz;
+    for (int a = 0; a < 3; ++a) {
+        d[a] = (x[a] - L.b[a] * L.dx) * L.inv_dx;
+        bspline1d(d[a], w[a], h[a]);
     }
 }
 
-template <int CZ, typename R>
-__device__ __forceinline__ void sweep_cell(const R* __restrict__ recs, const int* __restrict__ s_cs, int cb, int c0,
-                                           int c1, int g, const Piece<R>& px, const Piece<R>& py, R fi, R fj,
-                                           R* acc) {
-    const int lo = max(s_cs[cb + CZ], c0) - c0, hi = min(s_cs[cb + CZ + 1], c1) - c0;
-#pragma unroll 4
-    for (int p = lo; p < hi; ++p) accumulate<CZ>(recs + (size_t)p * kRec, g, px, py, fi, fj, acc);
+// acc += P_i (Y_j Z_k) + X_i (Y_j U_k + Q_j Z_k)
+template <typename R>
+__device__ __forceinline__ void add_terms(const pk_t<R> P[3], const pk_t<R> Q[3], const pk_t<R> U[3],
+                                          const R w[3][3], pk_t<R> acc[27]) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const pk_t<R> yz = dup<R>(w[1][j] * w[2][k]);
+            const pk_t<R> g = fma2(dup<R>(w[1][j]), U[k], mul2(Q[j], dup<R>(w[2][k])));
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                pk_t<R>& A = acc[i * 9 + j * 3 + k];
+                A = fma2(dup<R>(w[0][i]), g, fma2(P[i], yz, A));
+            }
+        }
 }
 
-// Channel of slot q (0..2) of group g's accumulator row.
-__device__ __forceinline__ int group_channel(int g, int q) {
-    if (q == 0) return CH_P0 + g;
-    if (q == 1) return g == 0 ? CH_M : (g == 1 ? CH_W : CH_VWFP);
-    return g == 0 ? CH_CW : (g == 1 ? CH_VW : CH_KC);
+// A lane's particles [lo, hi): o holds their previous slots, w0 the first one staged.  Loading the next particle's words
+// ahead was slower (730 against 715 us at 8.4M particles): the moves it takes cost more than the latency.
+template <typename R, int N, typename F>
+__device__ __forceinline__ void sweep(const R* stage, const int32_t* o, int w0, int lo, int hi, const int (&plane)[N],
+                                      F add) {
+#pragma unroll 1
+    for (int p = lo; p < hi; ++p) {
+        const R* s = stage + (o[p] - w0);
+        R v[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) v[q] = s[plane[q] * Staging<R>::WS];
+        add(v);
+    }
+}
+
+// Group 0: momentum x and y.
+template <typename R>
+__device__ __forceinline__ void add_momentum_xy(const R (&v)[17], const LaneCell<R>& L, pk_t<R> acc[27]) {
+    R d[3], w[3][3], h[3][3];
+    particle_weights(v, L, d, w, h);
+    const R m = v[3];
+    const pk_t<R> mD = dup<R>(m * L.kD);
+    // sigma rows x, y; stored xx yy zz xy xz yz.  B planes are column-major (r + 3c).
+    const R xx = L.kS * v[12], yy = L.kS * v[13], xy = L.kS * v[14], xz = L.kS * v[15], yz = L.kS * v[16];
+    const pk_t<R> sg[3] = {pk(xx, xy), pk(xy, yy), pk(xz, yz)};
+    pk_t<R> T[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const pk_t<R> b = mul2(mD, pk(v[6 + 2 * a], v[7 + 2 * a]));
+        pk_t<R> t = mul2(b, dup<R>(-d[a]));
+        if (a == 2) t = fma2(dup<R>(m), pk(v[4], v[5]), t);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            T[a][i] = fma2(t, dup<R>(w[a][i]), mul2(sg[a], dup<R>(h[a][i])));
+            if (i < 2) t = add2(t, b);
+        }
+    }
+    add_terms<R>(T[0], T[1], T[2], w, acc);
+}
+
+// Group 1: momentum z and the phase-field flux grad w . q.
+template <typename R>
+__device__ __forceinline__ void add_momentum_z_flux(const R (&v)[14], const LaneCell<R>& L, pk_t<R> acc[27]) {
+    R d[3], w[3][3], h[3][3];
+    particle_weights(v, L, d, w, h);
+    const R m = v[3];
+    const R mD = m * L.kD;
+    const pk_t<R> kk = pk(L.kS, L.inv_dx);
+    pk_t<R> T[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const pk_t<R> sg = mul2(kk, pk(v[8 + a], v[11 + a]));
+        const R b = mD * v[5 + a];
+        R t = -(b * d[a]);
+        if (a == 2) t += m * v[4];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            T[a][i] = mul2(sg, dup<R>(h[a][i]));
+            T[a][i].x += t * w[a][i];
+            if (i < 2) t += b;
+        }
+    }
+    add_terms<R>(T[0], T[1], T[2], w, acc);
+}
+
+// Group 2: mass and damage weight.
+template <typename R>
+__device__ __forceinline__ void add_mass_damage(const R (&v)[5], const LaneCell<R>& L, pk_t<R> acc[27]) {
+    R d[3], w[3][3], h[3][3];
+    particle_weights(v, L, d, w, h);
+    pk_t<R> X[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) X[i] = mul2(pk(v[3], v[4]), dup<R>(w[0][i]));
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const pk_t<R> yz = dup<R>(w[1][j] * w[2][k]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) acc[i * 9 + j * 3 + k] = fma2(X[i], yz, acc[i * 9 + j * 3 + k]);
+        }
+}
+
+// Group 3: weight and V w (pairs), V w FP.
+template <typename R>
+__device__ __forceinline__ void add_weights(const R (&v)[5], const LaneCell<R>& L, pk_t<R> acc[27], R one[27]) {
+    R d[3], w[3][3], h[3][3];
+    particle_weights(v, L, d, w, h);
+    const R V = v[3], VF = v[3] * v[4];
+    pk_t<R> X[3];
+    R X1[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        X[i] = pk(w[0][i], V * w[0][i]);
+        X1[i] = VF * w[0][i];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const R yz = w[1][j] * w[2][k];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const int q = i * 9 + j * 3 + k;
+                acc[q] = fma2(X[i], dup<R>(yz), acc[q]);
+                one[q] += X1[i] * yz;
+            }
+        }
 }
 
 // Chunk sequence of one CTA: its pages b + k g (b, g: the CTA's index and the
-// CTA count of its scene's share of the launch), each cut into runs of CH
+// CTA count of its scene's share of the launch), each cut into runs of kP2GChunk
 // slots.  Every thread runs the same iterator.
-template <int CH>
 struct ChunkIter {
     int page, next, end;  // current page, next run start, page end
     int nbs, nbe;         // slot range of the following page (loaded one page ahead)
@@ -279,8 +322,8 @@ struct ChunkIter {
         if (page < nb) {
             b = page;
             s0 = next;
-            n = min(CH, end - next);
-            next += CH;
+            n = min(kP2GChunk, end - next);
+            next += kP2GChunk;
             last = next >= end;
         } else {
             b = -1;
@@ -289,270 +332,313 @@ struct ChunkIter {
     }
 };
 
-template <int CH>
+
+// Cell sums of a page, [slot][stencil node][cell] pairs: slots 0..2 are groups
+// 0..2, slot 3 (W, V w), slot 4 (V w FP, 0).  The slot stride is padded so that
+// the five slots of a gathered column fall in different banks.
+constexpr int kSlots = 5;
+constexpr int kSlotStride = 27 * 64 + 2;
+constexpr int kItems = 36 * kSlots * 2;  // of the page gather
+// Tile channels of a slot's pair (-1: none).
+__device__ __forceinline__ int slot_channel(int slot, int half) {
+    const int c0 = slot == 0 ? CH_P0 : slot == 1 ? CH_P2 : slot == 2 ? CH_M : slot == 3 ? CH_W : CH_VWFP;
+    const int c1 = slot == 0 ? CH_P1 : slot == 1 ? CH_KC : slot == 2 ? CH_CW : slot == 3 ? CH_VW : -1;
+    return half == 0 ? c0 : c1;
+}
+// Window columns (a, b) as 6 a + b, by the number of cell columns that reach
+// them (9 6 4 3 2 1), so that a warp of the gather runs a similar number of terms.
+__constant__ unsigned char kColumnOrder[36] = {14, 15, 20, 21, 8,  9,  26, 27, 13, 16, 19, 22, 7,  10, 25, 28, 12, 17,
+                                               18, 23, 2,  3,  32, 33, 6,  11, 24, 29, 1,  4,  31, 34, 0,  5,  30, 35};
+
+template <typename R>
+__device__ __forceinline__ void set_lane_cell(LaneCell<R>& L, uint32_t page, int cell) {
+    int bx, by, bz;
+    page_coords(page, bx, by, bz);
+    L.b[0] = R(4 * bx + (cell >> 4));
+    L.b[1] = R(4 * by + ((cell >> 2) & 3));
+    L.b[2] = R(4 * bz + (cell & 3));
+}
+
+// Sums of a gather item (see make_item): three nodes of a window column, over
+// the cell columns that reach it.  A cell column's cells are added first, then
+// the columns along y, then (compensated) along x.  The upper half is the
+// mirror image: node 5 - z takes cell 3 - cz at stencil node 2 - k.
+constexpr int kNextY = 4 - 3 * 64, kNextX = 16 - 9 * 64;  // a node's sum in the next cell column along y, x
+template <typename P>
+__device__ __forceinline__ void gather_item(const P* __restrict__ sums, uint32_t w, P sum[3]) {
+    const int ni = (w >> 15) & 3, nj = (w >> 17) & 3;
+    const bool up = (w >> 19) & 1;
+    const int sk = up ? -64 : 64, sc = up ? -1 : 1;
+    const P* src = sums + (w & 0x7fff);
+    P comp[3];
+#pragma unroll
+    for (int z = 0; z < 3; ++z) sum[z].x = sum[z].y = comp[z].x = comp[z].y = 0;
+#pragma unroll 1
+    for (int i = 0; i < ni; ++i) {
+        P c0 = src[0], c1 = add2(src[sk], src[sc]), c2 = add2(add2(src[2 * sk], src[sk + sc]), src[2 * sc]);
+        const P* col = src;
+#pragma unroll 1
+        for (int j = 1; j < nj; ++j) {
+            col += kNextY;
+            c0 = add2(c0, col[0]);
+            c1 = add2(c1, add2(col[sk], col[sc]));
+            c2 = add2(c2, add2(add2(col[2 * sk], col[sk + sc]), col[2 * sc]));
+        }
+        kahan_add2(sum[0], comp[0], c0);
+        kahan_add2(sum[1], comp[1], c1);
+        kahan_add2(sum[2], comp[2], c2);
+        src += kNextX;
+    }
+}
+
+template <typename R>
 struct P2GMeta {
-    int32_t o[3][CH];     // previous slot per chunk slot; 3 buffers
-    uint32_t key[3][CH];  // sorted key per chunk slot
-    int32_t cs[3][68];    // cell starts of the chunk's page (65 used)
-    uint32_t bkey[3];
-    int32_t chunk[3][4];  // page, first slot, count (0: none), last chunk of page
-    int64_t win[3];       // first previous slot of the chunk's staging window
-    uint64_t bar;         // completion of the staging bulk copies
-    int abort;            // a bounded wait gave up
-    // page flush: the column-sum offsets of window node n's terms, in summing order
-    // (cell column cx then cy ascending), and their count
-    uint16_t goff[kWindowNodes][9];
-    uint8_t gcnt[kWindowNodes];
+    R tile[kP2GChannels * kWindowNodes];  // the page's gathered tile
+    int32_t o[2][kP2GChunk];              // previous slot per chunk slot; 2 buffers
+    int32_t cs[2][68];                    // cell starts of the chunk's page (65 used)
+    uint32_t bkey[2];
+    uint64_t bar;                         // completion of the staging bulk copies
+    const R* plane[kRawWords];            // raw planes in HBM
+    uint32_t item[kItems][2];             // gather items, built once per CTA (make_item)
+    int abort;                            // a bounded wait gave up
 };
+
+// A gather item: window column (a, b), slot and half of the column's six nodes.
+//   word 0: the first column's cell sum (bits 0-14), columns along x and y (15-16, 17-18), half (19)
+//   word 1: the item's first node in the tile, of the slot's first and second channel (bits 0-10, 16-26; 0xffff: none)
+__device__ __forceinline__ void make_item(int q, uint32_t w[2]) {
+    const int rank = q / (2 * kSlots), r = q - rank * 2 * kSlots;
+    const int slot = r >> 1, up = r & 1, col = kColumnOrder[rank];
+    const int a = col / 6, b = col - 6 * a;
+    // cell columns cx0 .. cx0 + ni - 1, cy0 .. cy0 + nj - 1, at stencil nodes (a - cx, b - cy)
+    const int cx0 = max(0, a - 2), ni = min(3, a) - cx0 + 1, cy0 = max(0, b - 2), nj = min(3, b) - cy0 + 1;
+    const int src = slot * kSlotStride + ((a - cx0) * 9 + (b - cy0) * 3) * 64 + cx0 * 16 + cy0 * 4;
+    w[0] = (uint32_t)(src + (up ? 2 * 64 + 3 : 0)) | (uint32_t)ni << 15 | (uint32_t)nj << 17 | (uint32_t)up << 19;
+    const int ch0 = slot_channel(slot, 0), ch1 = slot_channel(slot, 1), z = col * 6 + (up ? 5 : 0);
+    w[1] = (uint32_t)(ch0 * kWindowNodes + z) | ((uint32_t)(ch1 < 0 ? 0xffff : ch1 * kWindowNodes + z) << 16);
+}
 
 // Start of the staging window of a chunk: the median over three particles of
 // (previous slot - slot) estimates the chunk's shift between the orders.
-template <typename R, int CH>
 __device__ __forceinline__ int64_t window_start(const int32_t* o, int n, int64_t stride) {
     const int64_t d0 = o[0], d1 = (int64_t)o[n / 2] - n / 2, d2 = (int64_t)o[n - 1] - (n - 1);
     const int64_t med = max(min(d0, d1), min(max(d0, d1), d2));
     int64_t w = (med - kMargin) & ~(int64_t)3;
-    w = min(w, stride - Staging<R>::W);
+    w = min(w, stride - window_length(n));
     return max(w, (int64_t)0);
 }
 
-// Thread 0: bulk copies of the 28 raw planes over the chunk's window.
-template <typename R, int CH>
-__device__ __forceinline__ void issue_staging(P2GMeta<CH>& S, R* stage, int64_t w0, const PState<R>& st,
-                                              const PAux<R>& aux) {
-    constexpr int W = Staging<R>::W, WS = Staging<R>::WS;
-    fence_proxy_async_shared();
-    mbar_arrive_expect_tx(&S.bar, (unsigned)(kRawWords * W * sizeof(R)));
-#pragma unroll
-    for (int q = 0; q < kRawWords; ++q)
-        bulk_copy_g2s(stage + (size_t)q * WS, raw_plane(st, aux, q) + w0, (unsigned)(W * sizeof(R)), &S.bar);
-}
-
-template <int CH>
-__device__ __forceinline__ void issue_p2g_meta(P2GMeta<CH>& S, int m, int b, int s0, int n, const BinDev& bin) {
-    const int t = threadIdx.x;
-    if (n <= 0) return;
-    for (int p = t; p < n; p += kP2GThreads) {
-        cp_async_elem(&S.o[m][p], &bin.perm[s0 + p]);
-        cp_async_elem(&S.key[m][p], &bin.keys_sorted[s0 + p]);
-    }
-    if (t < 65) cp_async_elem(&S.cs[m][t], &bin.cell_start[(int64_t)b * 64 + t]);
-    if (t == 65) cp_async_elem(&S.bkey[m], &bin.block_keys[b]);
-}
-
+// Bulk copies of the raw planes over the chunk's window, a few planes per warp.
+// Called by one lane of every warp.
 template <typename R>
-constexpr size_t p2g_rec_bytes() {
-    return sizeof(R) * (size_t)P2GChunk<R>::value * kRec;
+__device__ __forceinline__ void issue_staging(const R* const* plane, uint64_t* bar, R* stage, int64_t w0, int len, int warp) {
+    constexpr int WS = Staging<R>::WS, kWarps = kP2GThreads / 32;
+    fence_proxy_async_shared();
+    const int planes = (kRawWords - warp + kWarps - 1) / kWarps;
+    mbar_arrive_expect_tx(bar, (unsigned)(planes * len * sizeof(R)));
+    for (int q = warp; q < kRawWords; q += kWarps)
+        bulk_copy_g2s(stage + (size_t)q * WS, plane[q] + w0, (unsigned)(len * sizeof(R)), bar);
 }
+
+// Slots, cell starts and key of a chunk.
+__device__ __forceinline__ void issue_p2g_meta(int32_t* o, int32_t* cs, uint32_t* bkey, int t, int b, int s0, int n,
+                                               const BinDev& bin) {
+    if (n <= 0) return;
+    for (int p = t; p < n; p += kP2GThreads) cp_async_elem(&o[p], &bin.perm[s0 + p]);
+    if (t < 65) cp_async_elem(&cs[t], &bin.cell_start[(int64_t)b * 64 + t]);
+    if (t == 65) cp_async_elem(bkey, &bin.block_keys[b]);
+}
+
+// Particles outside the window: gather the whole chunk into sorted order, in
+// place (a batch of planes is read by every thread before any is written), and
+// set the slots o to their new places.
+template <typename R>
+__device__ __forceinline__ void sort_staged(const R* const* plane, int32_t* o, R* stage, int n, int64_t w0, int len) {
+    const int t = threadIdx.x;
+    constexpr int kThreads = kP2GThreads;
+    constexpr int WS = Staging<R>::WS, kBatch = 4, kPer = (kP2GChunk + kThreads - 1) / kThreads;
+    static_assert(kRawWords % kBatch == 0, "whole batches");
+#pragma unroll 1
+    for (int qb = 0; qb < kRawWords; qb += kBatch) {
+        R v[kPer][kBatch];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int p = t + i * kThreads;
+            if (p >= n) continue;
+            const int64_t r = (int64_t)o[p] - w0;
+            if (r >= 0 && r < len) {
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) v[i][q] = stage[(size_t)(qb + q) * WS + r];
+            } else {
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) v[i][q] = plane[qb + q][o[p]];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int p = t + i * kThreads;
+            if (p >= n) continue;
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) stage[(size_t)(qb + q) * WS + p] = v[i][q];
+        }
+    }
+    for (int p = t; p < n; p += kThreads) o[p] = (int32_t)(w0 + p);
+    __syncthreads();
+}
+
 template <typename R>
 constexpr size_t p2g_stage_bytes() {
     return sizeof(R) * (size_t)kRawWords * Staging<R>::WS;
 }
+static_assert(2 * sizeof(float) * kSlots * kSlotStride <= p2g_stage_bytes<float>() &&
+                  2 * sizeof(double) * kSlots * kSlotStride <= p2g_stage_bytes<double>(),
+              "cell sums fit the staged planes");
 
-template <typename R, bool kDeterministic>
+template <typename R>
 __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ sc, const PState<R>& st,
                                          const PAux<R>& aux, const BinDev& bin, R* __restrict__ tile,
                                          Counters* __restrict__ cnt) {
-    constexpr int CH = P2GChunk<R>::value;
-    constexpr int W = Staging<R>::W, WS = Staging<R>::WS;
-    static_assert(sizeof(R) * kP2GChannels * kFlushChStride <= p2g_rec_bytes<R>(), "column sums fit the record buffer");
-    static_assert(sizeof(R) * kP2GChannels * kWindowNodes <= p2g_rec_bytes<R>(), "tile fits the record buffer");
+    using P2 = pk_t<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R* recs = reinterpret_cast<R*>(smem_raw);                          // [CH][kRec] particle records
-    R* stage = reinterpret_cast<R*>(smem_raw + p2g_rec_bytes<R>());   // [kRawWords][WS] raw planes
-    P2GMeta<CH>& S = *reinterpret_cast<P2GMeta<CH>*>(smem_raw + p2g_rec_bytes<R>() + p2g_stage_bytes<R>());
+    R* stage = reinterpret_cast<R*>(smem_raw);   // [kRawWords][WS] raw planes
+    P2* sums = reinterpret_cast<P2*>(smem_raw);  // the page's cell sums, once the planes are read
+    P2GMeta<R>& S = *reinterpret_cast<P2GMeta<R>*>(smem_raw + p2g_stage_bytes<R>());
 
     const int t = threadIdx.x;
     const int warp = t >> 5, lane = t & 31;
-    const int le = lane < 27 ? lane : lane - 27;  // lanes 27..31 shadow lanes 0..4 and never flush
-    const int g = le / 9;
-    const int col = le - g * 9;
-    const int ci = col / 3, cj = col - ci * 3;
-    // Warp w owns z-column (cx, cy) = (w / 4, (w - cx) mod 4): the four warps
-    // of a scheduler (w mod 4) then hold one column of every cx and every cy,
-    // so a page's empty rows or slabs of cells do not all land on one scheduler.
-    const int wcx = warp >> 2, wcy = ((warp & 3) - wcx) & 3;
-    const int cb = wcx * 16 + wcy * 4;  // first cell (cz = 0) of the z-column
-    const R inv_dx = sc->inv_dx;
-    const R fi = R(ci), fj = R(cj);
-    Piece<R> px, py;
-    px.init(ci, inv_dx);
-    py.init(cj, inv_dx);
+    // Two warps per group.  A scheduler (warp mod 4) holds one with the fuller and one with the lighter
+    // cells, of a momentum group and of a weight group.
+    const int group = (warp & 1) | ((warp >> 2) << 1);
+    const bool lighter = ((warp >> 1) & 1) != (warp >> 2);
     const int nb = min(cnt->n_blocks, bin.nb_cap);
+    LaneCell<R> L;
+    L.dx = sc->dx;
+    L.inv_dx = sc->inv_dx;
+    L.kD = sc->Dinv * sc->dx;
+    L.kS = -sc->dt * sc->inv_dx;
 
-    // prologue: meta of chunks 0 and 1, staging of chunk 0
-    ChunkIter<CH> it;
+    // prologue: descriptors of chunks 0 and 1, meta of chunk 0
+    ChunkIter it;
     it.init(bin, nb, vb);
-    {
-        int b0, s0, n0, l0, b1, s1, n1, l1;
-        it.step(bin, nb, b0, s0, n0, l0);
-        it.step(bin, nb, b1, s1, n1, l1);
-        if (t < kWindowNodes) {
-            const int na = t / 36, nbb = (t / 6) % 6, nc = t % 6;
-            int q = 0;
-            for (int cx = max(0, na - 2); cx <= min(3, na); ++cx)
-                for (int cy = max(0, nbb - 2); cy <= min(3, nbb); ++cy)
-                    S.goff[t][q++] = (uint16_t)(((cx * 4 + cy) * 9 + (na - cx) * 3 + (nbb - cy)) * 6 + nc);
-            S.gcnt[t] = (uint8_t)q;
-        }
-        if (t == 0) {
-            S.chunk[0][0] = b0; S.chunk[0][1] = s0; S.chunk[0][2] = n0; S.chunk[0][3] = l0;
-            S.chunk[1][0] = b1; S.chunk[1][1] = s1; S.chunk[1][2] = n1; S.chunk[1][3] = l1;
-            S.abort = 0;
-            mbar_init(&S.bar, 1);
-            mbar_init_fence();
-        }
-        issue_p2g_meta(S, 0, b0, s0, n0, bin);
-        cp_async_commit();
-        cp_async_wait_all();
-        __syncthreads();
-        if (t == 0 && n0 > 0) {
-            S.win[0] = window_start<R, CH>(S.o[0], n0, st.stride);
-            issue_staging(S, stage, S.win[0], st, aux);
-        }
-        issue_p2g_meta(S, 1, b1, s1, n1, bin);
-        cp_async_commit();
+    int b0, c0, n0, last0, b1, c1, n1, last1;
+    it.step(bin, nb, b0, c0, n0, last0);
+    it.step(bin, nb, b1, c1, n1, last1);
+    if (t == 0) {
+        S.abort = 0;
+        mbar_init(&S.bar, kP2GThreads / 32);
+        mbar_init_fence();
     }
-
-    R acc[18];
 #pragma unroll
-    for (int q = 0; q < 18; ++q) acc[q] = R(0);
+    for (int q = 0; q < kRawWords; ++q)
+        if (t == q) S.plane[q] = raw_plane(st, aux, q);
+    for (int q = t; q < kItems; q += kP2GThreads) make_item(q, S.item[q]);
+    issue_p2g_meta(S.o[0], S.cs[0], &S.bkey[0], t, b0, c0, n0, bin);
+    cp_async_commit();
+    bool first = true;  // first chunk of its page
+    int done = -1;      // page whose tile is ready to be written
 
     for (int k = 0;; ++k) {
-        const int m0 = k % 3, m1 = (k + 1) % 3, m2 = (k + 2) % 3;
+        const int m = k & 1;
         cp_async_wait_all();
-        const int n0 = S.chunk[m0][2];
-        if (n0 > 0 && !mbar_wait(&S.bar, (unsigned)(k & 1))) S.abort = 1;
+        // the sums and the tile were accessed by this thread; bulk copies follow
+        fence_proxy_async_shared();
         __syncthreads();
-        if (n0 <= 0 || S.abort) break;
-        const int b0 = S.chunk[m0][0], c0 = S.chunk[m0][1], last0 = S.chunk[m0][3];
-        // records of chunk k from the staged window (or directly for particles outside it)
-        {
-            int bx, by, bz;
-            page_coords(S.bkey[m0], bx, by, bz);
-            const int64_t w0 = S.win[m0];
-            for (int p = t; p < n0; p += kP2GThreads) {
-                const int o = S.o[m0][p];
-                const int64_t r = (int64_t)o - w0;
-                R raw[kRawWords];
-                if (r >= 0 && r < W) {
-#pragma unroll
-                    for (int q = 0; q < kRawWords; ++q) raw[q] = stage[(size_t)q * WS + r];
-                } else {
-#pragma unroll
-                    for (int q = 0; q < kRawWords; ++q) raw[q] = raw_plane(st, aux, q)[o];
-                }
-                const uint32_t cell = S.key[m0][p] & 63u;
-                const int base[3] = {4 * bx + (int)(cell >> 4), 4 * by + (int)((cell >> 2) & 3),
-                                     4 * bz + (int)(cell & 3)};
-                build_record(sc, base, raw, recs + (size_t)p * kRec);
-            }
+        if (t == 0 && done >= 0)
+            bulk_copy_s2g(tile + (int64_t)done * kP2GChannels * kWindowNodes, S.tile, (unsigned)sizeof(S.tile));
+        done = -1;
+        if (n0 <= 0) break;
+        const int64_t w0 = window_start(S.o[m], n0, st.stride);
+        const int len = window_length(n0);
+        if (lane == 0) issue_staging<R>(S.plane, &S.bar, stage, w0, len, warp);
+        issue_p2g_meta(S.o[m ^ 1], S.cs[m ^ 1], &S.bkey[m ^ 1], t, b1, c1, n1, bin);
+        cp_async_commit();
+        bool outside = false;
+        for (int p = t; p < n0; p += kP2GThreads) {
+            const int64_t r = (int64_t)S.o[m][p] - w0;
+            outside = outside || r < 0 || r >= len;
         }
-        __syncthreads();
+        // this lane's cell: the fuller (or, in the group's other warp, the lighter) of cells lane and lane + 32
+        int cell, lo, hi;
         {
-            // chunk k+1: staging (the buffer is free now); chunk k+2: iterator step, descriptor and meta.
-            // The staging copies are issued by the warp whose column holds the fewest of this chunk's
-            // particles, so that the issue delays the sweep least (each warp finds it the same way).
-            const int n1 = S.chunk[m1][2];
-            int issuer;
-            {
-                const int* cs = S.cs[m0];
-                const int c1 = c0 + n0;
-                const int lw = lane & 15;
-                const int lcx = lw >> 2, lcy = ((lw & 3) - lcx) & 3, lcb = lcx * 16 + lcy * 4;
-                int key = ((min(max(cs[lcb + 4], c0), c1) - min(max(cs[lcb], c0), c1)) << 4) | lw;
-#pragma unroll
-                for (int off = 8; off > 0; off >>= 1) key = min(key, __shfl_xor_sync(0xffffffffu, key, off));
-                issuer = key & 15;
-            }
-            if (warp == issuer && lane == 0 && n1 > 0) {
-                S.win[m1] = window_start<R, CH>(S.o[m1], n1, st.stride);
-                issue_staging(S, stage, S.win[m1], st, aux);
-            }
-            int b2, s2, n2, l2;
-            it.step(bin, nb, b2, s2, n2, l2);
-            if (t == 0) {
-                S.chunk[m2][0] = b2;
-                S.chunk[m2][1] = s2;
-                S.chunk[m2][2] = n2;
-                S.chunk[m2][3] = l2;
-            }
-            issue_p2g_meta(S, m2, b2, s2, n2, bin);
-            cp_async_commit();
+            const int* cs = S.cs[m];
+            const bool upper_fuller = cs[lane + 33] - cs[lane + 32] > cs[lane + 1] - cs[lane];
+            cell = upper_fuller != lighter ? lane + 32 : lane;
+            lo = max(cs[cell], c0) - c0;
+            hi = min(cs[cell + 1], c0 + n0) - c0;
+            set_lane_cell(L, S.bkey[m], cell);
         }
-        {
-            const int* s_cs = S.cs[m0];
-            const int c1 = c0 + n0;
-            sweep_cell<0>(recs, s_cs, cb, c0, c1, g, px, py, fi, fj, acc);
-            sweep_cell<1>(recs, s_cs, cb, c0, c1, g, px, py, fi, fj, acc);
-            sweep_cell<2>(recs, s_cs, cb, c0, c1, g, px, py, fi, fj, acc);
-            sweep_cell<3>(recs, s_cs, cb, c0, c1, g, px, py, fi, fj, acc);
-        }
-        if (!last0) continue;
+        if (!mbar_wait(&S.bar, (unsigned)m)) S.abort = 1;
+        outside = __syncthreads_or(outside);
+        if (S.abort) break;
+        if (outside) sort_staged<R>(S.plane, S.o[m], stage, n0, w0, len);
+        const int win = (int)w0;
 
-        // Page done: column sums -> the page's tile.  The sums go to the
-        // record buffer, which is free once every warp is past its sweep.
-        __syncthreads();
-        R* acc_smem = recs;
-        const int a = wcx + ci, bb = wcy + cj;
-        if (!kDeterministic) {
-            for (int q = t; q < kP2GChannels * kWindowNodes; q += kP2GThreads) acc_smem[q] = R(0);
-            __syncthreads();
-        }
-        if (lane < 27) {
+        // Cell sums.  Each group's sums stay in its own registers over the CTA's barrier, after which they
+        // overwrite the staged planes.
+        {
+            P2 acc[27];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const int ch = group_channel(g, q);
+            for (int q = 0; q < 27; ++q) acc[q] = pk(R(0), R(0));
+            P2* out = sums + group * kSlotStride + cell;
+            if (group == 0)
+                sweep<R>(stage, S.o[m], win, lo, hi, kWordsXY, [&](auto& v) { add_momentum_xy<R>(v, L, acc); });
+            else if (group == 1)
+                sweep<R>(stage, S.o[m], win, lo, hi, kWordsZQ, [&](auto& v) { add_momentum_z_flux<R>(v, L, acc); });
+            else if (group == 2)
+                sweep<R>(stage, S.o[m], win, lo, hi, kWordsMC, [&](auto& v) { add_mass_damage<R>(v, L, acc); });
+            if (group < 3) {
+                if (t == 0) bulk_store_wait_read();  // the previous tile has left shared memory
+                p2g_barrier();
 #pragma unroll
-                for (int z = 0; z < 6; ++z) {
-                    if (kDeterministic)
-                        acc_smem[ch * kFlushChStride + ((wcx * 4 + wcy) * 9 + col) * 6 + z] = acc[3 * z + q];
-                    else
-                        atomicAdd(&acc_smem[ch * kWindowNodes + a * 36 + bb * 6 + z], acc[3 * z + q]);
+                for (int q = 0; q < 27; ++q) out[q * 64] = acc[q];
+            } else {
+                R one[27];
+#pragma unroll
+                for (int q = 0; q < 27; ++q) one[q] = R(0);
+                sweep<R>(stage, S.o[m], win, lo, hi, kWordsV, [&](auto& v) { add_weights<R>(v, L, acc, one); });
+                p2g_barrier();
+#pragma unroll
+                for (int q = 0; q < 27; ++q) {
+                    out[q * 64] = acc[q];
+                    out[kSlotStride + q * 64] = pk(one[q], R(0));
                 }
             }
         }
-#pragma unroll
-        for (int q = 0; q < 18; ++q) acc[q] = R(0);
         __syncthreads();
-        R* out = tile + (int64_t)b0 * kP2GChannels * kWindowNodes;
-        if (kDeterministic) {
-            // tile value (ch, n): window node n = (a, b, c) sums cell columns (cx, cy) with stencil
-            // column (a - cx, b - cy), cx then cy ascending (compensated).  One (channel, node) sum per
-            // thread step over all threads: the sums are short dependent chains, so spreading them keeps
-            // every warp busy where one thread per node left most of the CTA waiting.
-            constexpr int kItems = (kP2GChannels * kWindowNodes + kP2GThreads - 1) / kP2GThreads;
-            int base[kItems], cnt[kItems];
-            R sum[kItems], comp[kItems];
+        // Gather: window column (a, b), slot and half of the column's six nodes per item.  A node sums its
+        // cell columns (cx, cy) = (a - i, b - j) in ascending order (compensated), each column's cells
+        // first.  The upper half is the mirror image: node 5 - z takes cell 3 - cz at stencil node 2 - k.
+        // Threads past the first 152 take a second, short item.
+        for (int it0 = t; it0 < kItems; it0 = it0 < kP2GThreads ? 2 * kP2GThreads - 1 - it0 : kItems) {
+            const uint32_t w0 = S.item[it0][0], w1 = S.item[it0][1];
+            P2 sum[3];
+            gather_item(sums, w0, sum);
+            R* t0 = S.tile + (w1 & 0xffff);
+            R* t1 = S.tile + (w1 >> 16);
+            const int dz = ((w0 >> 19) & 1) ? -1 : 1;
+            const bool two = (w1 >> 16) != 0xffff;
+            if (first) {
 #pragma unroll
-            for (int i = 0; i < kItems; ++i) {
-                const int w = t + i * kP2GThreads;
-                const int ch = w / kWindowNodes;
-                const int n = w - ch * kWindowNodes;
-                const bool ok = w < kP2GChannels * kWindowNodes;
-                base[i] = ok ? n * 9 : 0;
-                cnt[i] = ok ? S.gcnt[n] : 0;
-                sum[i] = comp[i] = R(0);
-                base[i] = (base[i] << 4) | ch;  // node's offset row and channel
+                for (int z = 0; z < 3; ++z) {
+                    t0[z * dz] = sum[z].x;
+                    if (two) t1[z * dz] = sum[z].y;
+                }
+            } else {
+#pragma unroll
+                for (int z = 0; z < 3; ++z) {
+                    t0[z * dz] += sum[z].x;
+                    if (two) t1[z * dz] += sum[z].y;
+                }
             }
-#pragma unroll
-            for (int q = 0; q < 9; ++q)
-#pragma unroll
-                for (int i = 0; i < kItems; ++i)
-                    if (q < cnt[i])
-                        kahan_add(sum[i], comp[i],
-                                  acc_smem[(base[i] & 15) * kFlushChStride + (&S.goff[0][0])[(base[i] >> 4) + q]]);
-#pragma unroll
-            for (int i = 0; i < kItems; ++i) {
-                const int w = t + i * kP2GThreads;
-                if (w < kP2GChannels * kWindowNodes) out[w] = sum[i];
-            }
-        } else {
-            for (int oi = t; oi < kP2GChannels * kWindowNodes; oi += kP2GThreads) out[oi] = acc_smem[oi];
         }
-        // The record buffer is rebuilt only after the next loop-top barrier.
+        if (last0) done = b0;
+        first = last0 != 0;
+        b0 = b1; c0 = c1; n0 = n1; last0 = last1;
+        it.step(bin, nb, b1, c1, n1, last1);
     }
     cp_async_wait_all();
+    if (t == 0) bulk_store_wait();
     if (S.abort) {
         // A staging copy may still be in flight: wait for it (bounded) before
         // the CTA's shared memory goes away, and report.
@@ -564,47 +650,46 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
     }
 }
 
-template <typename R, bool kDeterministic>
-__global__ void __launch_bounds__(kP2GThreads, 1)
+template <typename R>
+__global__ void __launch_bounds__(kP2GThreads, p2g_ctas_per_sm<R>())
     k_p2g(const SceneDev<R>* __restrict__ sc, PState<R> st, PAux<R> aux, BinDev bin, R* __restrict__ tile,
           Counters* __restrict__ cnt) {
-    p2g_body<R, kDeterministic>(own_blocks(), sc, st, aux, bin, tile, cnt);
+    p2g_body<R>(own_blocks(), sc, st, aux, bin, tile, cnt);
 }
 
 // Batched launch: the same body for the scene that owns this CTA.
-template <typename R, bool kDeterministic>
-__global__ void __launch_bounds__(kP2GThreads, 1)
+template <typename R>
+__global__ void __launch_bounds__(kP2GThreads, p2g_ctas_per_sm<R>())
     k_batch_p2g(const SceneArgs<R>* __restrict__ A, const int32_t* __restrict__ start, int ns) {
     VB vb;
     const SceneArgs<R>& a = A[scene_of_block(start, ns, vb)];
-    p2g_body<R, kDeterministic>(vb, a.sc, a.in, a.aux, a.bin, reinterpret_cast<R*>(a.grid.tile), a.cnt);
+    p2g_body<R>(vb, a.sc, a.in, a.aux, a.bin, reinterpret_cast<R*>(a.grid.tile), a.cnt);
 }
 
 template <typename R>
 size_t p2g_smem_bytes() {
-    return p2g_rec_bytes<R>() + p2g_stage_bytes<R>() + sizeof(P2GMeta<P2GChunk<R>::value>);
+    return p2g_stage_bytes<R>() + sizeof(P2GMeta<R>);
 }
 
 template <typename R>
 cudaError_t prepare_p2g() {
     const int smem = (int)p2g_smem_bytes<R>();
-    cudaError_t e = cudaFuncSetAttribute(k_p2g<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_p2g<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_batch_p2g<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_batch_p2g<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(k_p2g<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch_p2g<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     return e;
 }
 
 template <typename R>
+int p2g_ctas(int nb_cap, int sms) {
+    return max(1, min(nb_cap, sms * p2g_ctas_per_sm<R>()));
+}
+template int p2g_ctas<float>(int, int);
+template int p2g_ctas<double>(int, int);
+
+template <typename R>
 cudaError_t launch_batch_p2g(const SceneArgs<R>* A, const BatchPlan& P, cudaStream_t s) {
-    const dim3 grid((unsigned)P.total[BM_P2G]);
-    if (P.deterministic)
-        return launch_kernel(k_batch_p2g<R, true>, grid, dim3(kP2GThreads), p2g_smem_bytes<R>(), s, A, P.start[BM_P2G],
-                             P.n_scenes);
-    return launch_kernel(k_batch_p2g<R, false>, grid, dim3(kP2GThreads), p2g_smem_bytes<R>(), s, A, P.start[BM_P2G],
-                         P.n_scenes);
+    return launch_kernel(k_batch_p2g<R>, dim3((unsigned)P.total[BM_P2G]), dim3(kP2GThreads), p2g_smem_bytes<R>(), s, A,
+                         P.start[BM_P2G], P.n_scenes);
 }
 template cudaError_t launch_batch_p2g<float>(const SceneArgs<float>*, const BatchPlan&, cudaStream_t);
 template cudaError_t launch_batch_p2g<double>(const SceneArgs<double>*, const BatchPlan&, cudaStream_t);
@@ -614,12 +699,8 @@ template cudaError_t prepare_p2g<double>();
 template <typename R>
 cudaError_t launch_p2g(const SceneDev<R>* sc, const PState<R>& st, const PAux<R>& aux, BinDev bin, GridDev grid,
                        Counters* cnt, LaunchCfg cfg, cudaStream_t stream) {
-    const int ctas = max(1, min(bin.nb_cap, cfg.num_sms));
-    R* tile = reinterpret_cast<R*>(grid.tile);
-    if (cfg.deterministic)
-        k_p2g<R, true><<<ctas, kP2GThreads, p2g_smem_bytes<R>(), stream>>>(sc, st, aux, bin, tile, cnt);
-    else
-        k_p2g<R, false><<<ctas, kP2GThreads, p2g_smem_bytes<R>(), stream>>>(sc, st, aux, bin, tile, cnt);
+    k_p2g<R><<<p2g_ctas<R>(bin.nb_cap, cfg.num_sms), kP2GThreads, p2g_smem_bytes<R>(), stream>>>(
+        sc, st, aux, bin, reinterpret_cast<R*>(grid.tile), cnt);
     return cudaGetLastError();
 }
 
