@@ -40,46 +40,24 @@
 // memory 49%.  Measured on FP32 plates: 0.718 ms at 8.4M particles and 2.73 ms
 // at 33.5M, where one lane per stencil column, all lanes on the same particle,
 // took 1.209 and 4.67 (88 warp instructions a particle against 51: every
-// particle's words were read, and its weights formed, by 27 lanes).  FP64 at
-// 1.1M particles: 0.245 against 0.391 ms.
+// particle's words were read, and its weights formed, by 27 lanes).
 #include <cstdint>
 
-#include "async_copy.cuh"
-#include "kernels.h"
 #include "launch.cuh"
+#include "p2g_common.cuh"
 
 namespace gmpm {
+namespace {
+
+using R = float;
 
 constexpr int kP2GGroups = 4;
 constexpr int kP2GThreads = 64 * kP2GGroups;  // two warps (64 cells) per channel group
 constexpr int kP2GChunk = 576;
-template <typename R>
-constexpr int p2g_ctas_per_sm() { return sizeof(R) == 4 ? 2 : 1; }  // by registers and shared memory
-
-// Raw particle planes, in staging order.
-enum RawField : int {
-    RW_X = 0, RW_V = 3, RW_B = 6, RW_SIG = 15, RW_C = 21, RW_M = 22, RW_VOL = 23, RW_FP = 24, RW_Q = 25,
-    kRawWords = 28
-};
-
-// Device pointer of raw plane q.
-template <typename R>
-__device__ __forceinline__ const R* raw_plane(const PState<R>& st, const PAux<R>& aux, int q) {
-    if (q < RW_V) return st.x[q - RW_X];
-    if (q < RW_B) return aux.v[q - RW_V];
-    if (q < RW_SIG) return aux.B[q - RW_B];
-    if (q < RW_C) return aux.sigma[q - RW_SIG];
-    if (q == RW_C) return st.c;
-    if (q == RW_M) return st.m;
-    if (q == RW_VOL) return aux.vol;
-    if (q == RW_FP) return aux.FP;
-    return aux.q[q - RW_Q];
-}
+constexpr int kCtasPerSm = 2;  // by registers and shared memory
 
 // Staging window of previous slots: the chunk's slots plus kMargin on either
 // side; planes padded in shared memory to spread banks.
-constexpr int kMargin = 64;
-template <typename R>
 struct Staging {
     static constexpr int W = kP2GChunk + 2 * kMargin;      // longest window (elements)
     static constexpr int WS = W + (int)(16 / sizeof(R));   // plane stride in shared memory
@@ -88,27 +66,16 @@ struct Staging {
 };
 __device__ __forceinline__ int window_length(int n) { return (n + 2 * kMargin + 3) & ~3; }
 
-// Two channels of one value.  FP32: Blackwell's packed instructions.
-template <typename R> struct Pk;
-template <> struct Pk<float> { using T = float2; };
-template <> struct Pk<double> { using T = double2; };
-template <typename R> using pk_t = typename Pk<R>::T;
-__device__ __forceinline__ float2 pk(float a, float b) { return make_float2(a, b); }
-__device__ __forceinline__ double2 pk(double a, double b) { return make_double2(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
-    return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-template <typename R>
-__device__ __forceinline__ pk_t<R> dup(R a) { return pk(a, a); }
+// Two channels of one value, for Blackwell's packed FP32 instructions.
+using P2 = float2;
+__device__ __forceinline__ P2 pk(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ P2 dup(float a) { return make_float2(a, a); }
+__device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ P2 mul2(P2 a, P2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ P2 add2(P2 a, P2 b) { return __fadd2_rn(a, b); }
 
 // quadratic B-spline weights on nodes base+0..2 and their gradients times dx,
 // d = (x - x_base) / dx (P2GKernal.cu:590-611)
-template <typename R>
 __device__ __forceinline__ void bspline1d(R d, R* w, R* h) {
     const R z0 = R(1.5) - d, z1 = d - R(1), z2 = d - R(0.5);
     w[0] = R(0.5) * z0 * z0;
@@ -119,11 +86,10 @@ __device__ __forceinline__ void bspline1d(R d, R* w, R* h) {
     h[2] = z2;
 }
 
-template <typename P>
-__device__ __forceinline__ void kahan_add2(P& s, P& c, P v) {
-    const P minus = pk(decltype(s.x)(-1), decltype(s.x)(-1));
-    const P y = fma2(c, minus, v);
-    const P t = add2(s, y);
+__device__ __forceinline__ void kahan_add2(P2& s, P2& c, P2 v) {
+    const P2 minus = dup(R(-1));
+    const P2 y = fma2(c, minus, v);
+    const P2 t = add2(s, y);
     c = fma2(y, minus, fma2(s, minus, t));
     s = t;
 }
@@ -134,7 +100,6 @@ __device__ __forceinline__ void p2g_barrier() {
 }
 
 // What a lane keeps about its cell and the scene.
-template <typename R>
 struct LaneCell {
     R b[3];           // base node coordinates
     R dx, inv_dx, kD, kS;  // kD = dx D^-1, kS = -dt / dx
@@ -149,8 +114,7 @@ __device__ constexpr int kWordsZQ[14] = {RW_X,     RW_X + 1, RW_X + 2,   RW_M,  
 __device__ constexpr int kWordsMC[5] = {RW_X, RW_X + 1, RW_X + 2, RW_M, RW_C};
 __device__ constexpr int kWordsV[5] = {RW_X, RW_X + 1, RW_X + 2, RW_VOL, RW_FP};
 
-template <typename R>
-__device__ __forceinline__ void particle_weights(const R* x, const LaneCell<R>& L, R d[3], R w[3][3], R h[3][3]) {
+__device__ __forceinline__ void particle_weights(const R* x, const LaneCell& L, R d[3], R w[3][3], R h[3][3]) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         d[a] = (x[a] - L.b[a] * L.dx) * L.inv_dx;
@@ -159,26 +123,25 @@ __device__ __forceinline__ void particle_weights(const R* x, const LaneCell<R>& 
 }
 
 // acc += P_i (Y_j Z_k) + X_i (Y_j U_k + Q_j Z_k)
-template <typename R>
-__device__ __forceinline__ void add_terms(const pk_t<R> P[3], const pk_t<R> Q[3], const pk_t<R> U[3],
-                                          const R w[3][3], pk_t<R> acc[27]) {
+__device__ __forceinline__ void add_terms(const P2 P[3], const P2 Q[3], const P2 U[3],
+                                          const R w[3][3], P2 acc[27]) {
 #pragma unroll
     for (int j = 0; j < 3; ++j)
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const pk_t<R> yz = dup<R>(w[1][j] * w[2][k]);
-            const pk_t<R> g = fma2(dup<R>(w[1][j]), U[k], mul2(Q[j], dup<R>(w[2][k])));
+            const P2 yz = dup(w[1][j] * w[2][k]);
+            const P2 g = fma2(dup(w[1][j]), U[k], mul2(Q[j], dup(w[2][k])));
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                pk_t<R>& A = acc[i * 9 + j * 3 + k];
-                A = fma2(dup<R>(w[0][i]), g, fma2(P[i], yz, A));
+                P2& A = acc[i * 9 + j * 3 + k];
+                A = fma2(dup(w[0][i]), g, fma2(P[i], yz, A));
             }
         }
 }
 
 // A lane's particles [lo, hi): o holds their previous slots, w0 the first one staged.  Loading the next particle's words
 // ahead was slower (730 against 715 us at 8.4M particles): the moves it takes cost more than the latency.
-template <typename R, int N, typename F>
+template <int N, typename F>
 __device__ __forceinline__ void sweep(const R* stage, const int32_t* o, int w0, int lo, int hi, const int (&plane)[N],
                                       F add) {
 #pragma unroll 1
@@ -186,86 +149,82 @@ __device__ __forceinline__ void sweep(const R* stage, const int32_t* o, int w0, 
         const R* s = stage + (o[p] - w0);
         R v[N];
 #pragma unroll
-        for (int q = 0; q < N; ++q) v[q] = s[plane[q] * Staging<R>::WS];
+        for (int q = 0; q < N; ++q) v[q] = s[plane[q] * Staging::WS];
         add(v);
     }
 }
 
 // Group 0: momentum x and y.
-template <typename R>
-__device__ __forceinline__ void add_momentum_xy(const R (&v)[17], const LaneCell<R>& L, pk_t<R> acc[27]) {
+__device__ __forceinline__ void add_momentum_xy(const R (&v)[17], const LaneCell& L, P2 acc[27]) {
     R d[3], w[3][3], h[3][3];
     particle_weights(v, L, d, w, h);
     const R m = v[3];
-    const pk_t<R> mD = dup<R>(m * L.kD);
+    const P2 mD = dup(m * L.kD);
     // sigma rows x, y; stored xx yy zz xy xz yz.  B planes are column-major (r + 3c).
     const R xx = L.kS * v[12], yy = L.kS * v[13], xy = L.kS * v[14], xz = L.kS * v[15], yz = L.kS * v[16];
-    const pk_t<R> sg[3] = {pk(xx, xy), pk(xy, yy), pk(xz, yz)};
-    pk_t<R> T[3][3];
+    const P2 sg[3] = {pk(xx, xy), pk(xy, yy), pk(xz, yz)};
+    P2 T[3][3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const pk_t<R> b = mul2(mD, pk(v[6 + 2 * a], v[7 + 2 * a]));
-        pk_t<R> t = mul2(b, dup<R>(-d[a]));
-        if (a == 2) t = fma2(dup<R>(m), pk(v[4], v[5]), t);
+        const P2 b = mul2(mD, pk(v[6 + 2 * a], v[7 + 2 * a]));
+        P2 t = mul2(b, dup(-d[a]));
+        if (a == 2) t = fma2(dup(m), pk(v[4], v[5]), t);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            T[a][i] = fma2(t, dup<R>(w[a][i]), mul2(sg[a], dup<R>(h[a][i])));
+            T[a][i] = fma2(t, dup(w[a][i]), mul2(sg[a], dup(h[a][i])));
             if (i < 2) t = add2(t, b);
         }
     }
-    add_terms<R>(T[0], T[1], T[2], w, acc);
+    add_terms(T[0], T[1], T[2], w, acc);
 }
 
 // Group 1: momentum z and the phase-field flux grad w . q.
-template <typename R>
-__device__ __forceinline__ void add_momentum_z_flux(const R (&v)[14], const LaneCell<R>& L, pk_t<R> acc[27]) {
+__device__ __forceinline__ void add_momentum_z_flux(const R (&v)[14], const LaneCell& L, P2 acc[27]) {
     R d[3], w[3][3], h[3][3];
     particle_weights(v, L, d, w, h);
     const R m = v[3];
     const R mD = m * L.kD;
-    const pk_t<R> kk = pk(L.kS, L.inv_dx);
-    pk_t<R> T[3][3];
+    const P2 kk = pk(L.kS, L.inv_dx);
+    P2 T[3][3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const pk_t<R> sg = mul2(kk, pk(v[8 + a], v[11 + a]));
+        const P2 sg = mul2(kk, pk(v[8 + a], v[11 + a]));
         const R b = mD * v[5 + a];
         R t = -(b * d[a]);
         if (a == 2) t += m * v[4];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            T[a][i] = mul2(sg, dup<R>(h[a][i]));
+            T[a][i] = mul2(sg, dup(h[a][i]));
             T[a][i].x += t * w[a][i];
             if (i < 2) t += b;
         }
     }
-    add_terms<R>(T[0], T[1], T[2], w, acc);
+    add_terms(T[0], T[1], T[2], w, acc);
 }
 
 // Group 2: mass and damage weight.
-template <typename R>
-__device__ __forceinline__ void add_mass_damage(const R (&v)[5], const LaneCell<R>& L, pk_t<R> acc[27]) {
+__device__ __forceinline__ void add_mass_damage(const R (&v)[5], const LaneCell& L, P2 acc[27]) {
     R d[3], w[3][3], h[3][3];
     particle_weights(v, L, d, w, h);
-    pk_t<R> X[3];
+    P2 X[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) X[i] = mul2(pk(v[3], v[4]), dup<R>(w[0][i]));
+    for (int i = 0; i < 3; ++i) X[i] = mul2(pk(v[3], v[4]), dup(w[0][i]));
 #pragma unroll
     for (int j = 0; j < 3; ++j)
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const pk_t<R> yz = dup<R>(w[1][j] * w[2][k]);
+            const P2 yz = dup(w[1][j] * w[2][k]);
 #pragma unroll
             for (int i = 0; i < 3; ++i) acc[i * 9 + j * 3 + k] = fma2(X[i], yz, acc[i * 9 + j * 3 + k]);
         }
 }
 
 // Group 3: weight and V w (pairs), V w FP.
-template <typename R>
-__device__ __forceinline__ void add_weights(const R (&v)[5], const LaneCell<R>& L, pk_t<R> acc[27], R one[27]) {
+__device__ __forceinline__ void add_weights(const R (&v)[5], const LaneCell& L, P2 acc[27], R one[27]) {
     R d[3], w[3][3], h[3][3];
     particle_weights(v, L, d, w, h);
     const R V = v[3], VF = v[3] * v[4];
-    pk_t<R> X[3];
+    P2 X[3];
     R X1[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -280,58 +239,11 @@ __device__ __forceinline__ void add_weights(const R (&v)[5], const LaneCell<R>& 
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 const int q = i * 9 + j * 3 + k;
-                acc[q] = fma2(X[i], dup<R>(yz), acc[q]);
+                acc[q] = fma2(X[i], dup(yz), acc[q]);
                 one[q] += X1[i] * yz;
             }
         }
 }
-
-// Chunk sequence of one CTA: its pages b + k g (b, g: the CTA's index and the
-// CTA count of its scene's share of the launch), each cut into runs of kP2GChunk
-// slots.  Every thread runs the same iterator.
-struct ChunkIter {
-    int page, next, end;  // current page, next run start, page end
-    int nbs, nbe;         // slot range of the following page (loaded one page ahead)
-    int stride;           // CTAs of the scene's share of the launch
-    __device__ void init(const BinDev& bin, int nb, VB vb) {
-        page = vb.b;
-        stride = vb.g;
-        next = end = 0;
-        if (page < nb) {
-            next = bin.cell_start[(int64_t)page * 64];
-            end = bin.cell_start[(int64_t)page * 64 + 64];
-        }
-        preload(bin, nb);
-    }
-    __device__ void preload(const BinDev& bin, int nb) {
-        const int q = page + stride;
-        nbs = nbe = 0;
-        if (q < nb) {
-            nbs = bin.cell_start[(int64_t)q * 64];
-            nbe = bin.cell_start[(int64_t)q * 64 + 64];
-        }
-    }
-    // Next chunk (page, first slot, count, last chunk of its page); count 0 when done.
-    __device__ void step(const BinDev& bin, int nb, int& b, int& s0, int& n, int& last) {
-        while (page < nb && next >= end) {
-            page += stride;
-            next = nbs;
-            end = nbe;
-            if (page < nb) preload(bin, nb);
-        }
-        if (page < nb) {
-            b = page;
-            s0 = next;
-            n = min(kP2GChunk, end - next);
-            next += kP2GChunk;
-            last = next >= end;
-        } else {
-            b = -1;
-            s0 = n = last = 0;
-        }
-    }
-};
-
 
 // Cell sums of a page, [slot][stencil node][cell] pairs: slots 0..2 are groups
 // 0..2, slot 3 (W, V w), slot 4 (V w FP, 0).  The slot stride is padded so that
@@ -350,8 +262,7 @@ __device__ __forceinline__ int slot_channel(int slot, int half) {
 __constant__ unsigned char kColumnOrder[36] = {14, 15, 20, 21, 8,  9,  26, 27, 13, 16, 19, 22, 7,  10, 25, 28, 12, 17,
                                                18, 23, 2,  3,  32, 33, 6,  11, 24, 29, 1,  4,  31, 34, 0,  5,  30, 35};
 
-template <typename R>
-__device__ __forceinline__ void set_lane_cell(LaneCell<R>& L, uint32_t page, int cell) {
+__device__ __forceinline__ void set_lane_cell(LaneCell& L, uint32_t page, int cell) {
     int bx, by, bz;
     page_coords(page, bx, by, bz);
     L.b[0] = R(4 * bx + (cell >> 4));
@@ -364,19 +275,18 @@ __device__ __forceinline__ void set_lane_cell(LaneCell<R>& L, uint32_t page, int
 // the columns along y, then (compensated) along x.  The upper half is the
 // mirror image: node 5 - z takes cell 3 - cz at stencil node 2 - k.
 constexpr int kNextY = 4 - 3 * 64, kNextX = 16 - 9 * 64;  // a node's sum in the next cell column along y, x
-template <typename P>
-__device__ __forceinline__ void gather_item(const P* __restrict__ sums, uint32_t w, P sum[3]) {
+__device__ __forceinline__ void gather_item(const P2* __restrict__ sums, uint32_t w, P2 sum[3]) {
     const int ni = (w >> 15) & 3, nj = (w >> 17) & 3;
     const bool up = (w >> 19) & 1;
     const int sk = up ? -64 : 64, sc = up ? -1 : 1;
-    const P* src = sums + (w & 0x7fff);
-    P comp[3];
+    const P2* src = sums + (w & 0x7fff);
+    P2 comp[3];
 #pragma unroll
     for (int z = 0; z < 3; ++z) sum[z].x = sum[z].y = comp[z].x = comp[z].y = 0;
 #pragma unroll 1
     for (int i = 0; i < ni; ++i) {
-        P c0 = src[0], c1 = add2(src[sk], src[sc]), c2 = add2(add2(src[2 * sk], src[sk + sc]), src[2 * sc]);
-        const P* col = src;
+        P2 c0 = src[0], c1 = add2(src[sk], src[sc]), c2 = add2(add2(src[2 * sk], src[sk + sc]), src[2 * sc]);
+        const P2* col = src;
 #pragma unroll 1
         for (int j = 1; j < nj; ++j) {
             col += kNextY;
@@ -391,7 +301,6 @@ __device__ __forceinline__ void gather_item(const P* __restrict__ sums, uint32_t
     }
 }
 
-template <typename R>
 struct P2GMeta {
     R tile[kP2GChannels * kWindowNodes];  // the page's gathered tile
     int32_t o[2][kP2GChunk];              // previous slot per chunk slot; 2 buffers
@@ -418,21 +327,10 @@ __device__ __forceinline__ void make_item(int q, uint32_t w[2]) {
     w[1] = (uint32_t)(ch0 * kWindowNodes + z) | ((uint32_t)(ch1 < 0 ? 0xffff : ch1 * kWindowNodes + z) << 16);
 }
 
-// Start of the staging window of a chunk: the median over three particles of
-// (previous slot - slot) estimates the chunk's shift between the orders.
-__device__ __forceinline__ int64_t window_start(const int32_t* o, int n, int64_t stride) {
-    const int64_t d0 = o[0], d1 = (int64_t)o[n / 2] - n / 2, d2 = (int64_t)o[n - 1] - (n - 1);
-    const int64_t med = max(min(d0, d1), min(max(d0, d1), d2));
-    int64_t w = (med - kMargin) & ~(int64_t)3;
-    w = min(w, stride - window_length(n));
-    return max(w, (int64_t)0);
-}
-
 // Bulk copies of the raw planes over the chunk's window, a few planes per warp.
 // Called by one lane of every warp.
-template <typename R>
 __device__ __forceinline__ void issue_staging(const R* const* plane, uint64_t* bar, R* stage, int64_t w0, int len, int warp) {
-    constexpr int WS = Staging<R>::WS, kWarps = kP2GThreads / 32;
+    constexpr int WS = Staging::WS, kWarps = kP2GThreads / 32;
     fence_proxy_async_shared();
     const int planes = (kRawWords - warp + kWarps - 1) / kWarps;
     mbar_arrive_expect_tx(bar, (unsigned)(planes * len * sizeof(R)));
@@ -452,11 +350,10 @@ __device__ __forceinline__ void issue_p2g_meta(int32_t* o, int32_t* cs, uint32_t
 // Particles outside the window: gather the whole chunk into sorted order, in
 // place (a batch of planes is read by every thread before any is written), and
 // set the slots o to their new places.
-template <typename R>
 __device__ __forceinline__ void sort_staged(const R* const* plane, int32_t* o, R* stage, int n, int64_t w0, int len) {
     const int t = threadIdx.x;
     constexpr int kThreads = kP2GThreads;
-    constexpr int WS = Staging<R>::WS, kBatch = 4, kPer = (kP2GChunk + kThreads - 1) / kThreads;
+    constexpr int WS = Staging::WS, kBatch = 4, kPer = (kP2GChunk + kThreads - 1) / kThreads;
     static_assert(kRawWords % kBatch == 0, "whole batches");
 #pragma unroll 1
     for (int qb = 0; qb < kRawWords; qb += kBatch) {
@@ -487,23 +384,18 @@ __device__ __forceinline__ void sort_staged(const R* const* plane, int32_t* o, R
     __syncthreads();
 }
 
-template <typename R>
 constexpr size_t p2g_stage_bytes() {
-    return sizeof(R) * (size_t)kRawWords * Staging<R>::WS;
+    return sizeof(R) * (size_t)kRawWords * Staging::WS;
 }
-static_assert(2 * sizeof(float) * kSlots * kSlotStride <= p2g_stage_bytes<float>() &&
-                  2 * sizeof(double) * kSlots * kSlotStride <= p2g_stage_bytes<double>(),
-              "cell sums fit the staged planes");
+static_assert(2 * sizeof(float) * kSlots * kSlotStride <= p2g_stage_bytes(), "cell sums fit the staged planes");
 
-template <typename R>
 __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ sc, const PState<R>& st,
                                          const PAux<R>& aux, const BinDev& bin, R* __restrict__ tile,
                                          Counters* __restrict__ cnt) {
-    using P2 = pk_t<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* stage = reinterpret_cast<R*>(smem_raw);   // [kRawWords][WS] raw planes
     P2* sums = reinterpret_cast<P2*>(smem_raw);  // the page's cell sums, once the planes are read
-    P2GMeta<R>& S = *reinterpret_cast<P2GMeta<R>*>(smem_raw + p2g_stage_bytes<R>());
+    P2GMeta& S = *reinterpret_cast<P2GMeta*>(smem_raw + p2g_stage_bytes());
 
     const int t = threadIdx.x;
     const int warp = t >> 5, lane = t & 31;
@@ -512,14 +404,14 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
     const int group = (warp & 1) | ((warp >> 2) << 1);
     const bool lighter = ((warp >> 1) & 1) != (warp >> 2);
     const int nb = min(cnt->n_blocks, bin.nb_cap);
-    LaneCell<R> L;
+    LaneCell L;
     L.dx = sc->dx;
     L.inv_dx = sc->inv_dx;
     L.kD = sc->Dinv * sc->dx;
     L.kS = -sc->dt * sc->inv_dx;
 
     // prologue: descriptors of chunks 0 and 1, meta of chunk 0
-    ChunkIter it;
+    ChunkIter<kP2GChunk> it;
     it.init(bin, nb, vb);
     int b0, c0, n0, last0, b1, c1, n1, last1;
     it.step(bin, nb, b0, c0, n0, last0);
@@ -548,9 +440,9 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
             bulk_copy_s2g(tile + (int64_t)done * kP2GChannels * kWindowNodes, S.tile, (unsigned)sizeof(S.tile));
         done = -1;
         if (n0 <= 0) break;
-        const int64_t w0 = window_start(S.o[m], n0, st.stride);
         const int len = window_length(n0);
-        if (lane == 0) issue_staging<R>(S.plane, &S.bar, stage, w0, len, warp);
+        const int64_t w0 = window_start(S.o[m], n0, st.stride, len);
+        if (lane == 0) issue_staging(S.plane, &S.bar, stage, w0, len, warp);
         issue_p2g_meta(S.o[m ^ 1], S.cs[m ^ 1], &S.bkey[m ^ 1], t, b1, c1, n1, bin);
         cp_async_commit();
         bool outside = false;
@@ -571,7 +463,7 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
         if (!mbar_wait(&S.bar, (unsigned)m)) S.abort = 1;
         outside = __syncthreads_or(outside);
         if (S.abort) break;
-        if (outside) sort_staged<R>(S.plane, S.o[m], stage, n0, w0, len);
+        if (outside) sort_staged(S.plane, S.o[m], stage, n0, w0, len);
         const int win = (int)w0;
 
         // Cell sums.  Each group's sums stay in its own registers over the CTA's barrier, after which they
@@ -582,11 +474,11 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
             for (int q = 0; q < 27; ++q) acc[q] = pk(R(0), R(0));
             P2* out = sums + group * kSlotStride + cell;
             if (group == 0)
-                sweep<R>(stage, S.o[m], win, lo, hi, kWordsXY, [&](auto& v) { add_momentum_xy<R>(v, L, acc); });
+                sweep(stage, S.o[m], win, lo, hi, kWordsXY, [&](auto& v) { add_momentum_xy(v, L, acc); });
             else if (group == 1)
-                sweep<R>(stage, S.o[m], win, lo, hi, kWordsZQ, [&](auto& v) { add_momentum_z_flux<R>(v, L, acc); });
+                sweep(stage, S.o[m], win, lo, hi, kWordsZQ, [&](auto& v) { add_momentum_z_flux(v, L, acc); });
             else if (group == 2)
-                sweep<R>(stage, S.o[m], win, lo, hi, kWordsMC, [&](auto& v) { add_mass_damage<R>(v, L, acc); });
+                sweep(stage, S.o[m], win, lo, hi, kWordsMC, [&](auto& v) { add_mass_damage(v, L, acc); });
             if (group < 3) {
                 if (t == 0) bulk_store_wait_read();  // the previous tile has left shared memory
                 p2g_barrier();
@@ -596,7 +488,7 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
                 R one[27];
 #pragma unroll
                 for (int q = 0; q < 27; ++q) one[q] = R(0);
-                sweep<R>(stage, S.o[m], win, lo, hi, kWordsV, [&](auto& v) { add_weights<R>(v, L, acc, one); });
+                sweep(stage, S.o[m], win, lo, hi, kWordsV, [&](auto& v) { add_weights(v, L, acc, one); });
                 p2g_barrier();
 #pragma unroll
                 for (int q = 0; q < 27; ++q) {
@@ -650,63 +542,48 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
     }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(kP2GThreads, p2g_ctas_per_sm<R>())
+__global__ void __launch_bounds__(kP2GThreads, kCtasPerSm)
     k_p2g(const SceneDev<R>* __restrict__ sc, PState<R> st, PAux<R> aux, BinDev bin, R* __restrict__ tile,
-          Counters* __restrict__ cnt) {
-    p2g_body<R>(own_blocks(), sc, st, aux, bin, tile, cnt);
+            Counters* __restrict__ cnt) {
+    p2g_body(own_blocks(), sc, st, aux, bin, tile, cnt);
 }
 
 // Batched launch: the same body for the scene that owns this CTA.
-template <typename R>
-__global__ void __launch_bounds__(kP2GThreads, p2g_ctas_per_sm<R>())
+__global__ void __launch_bounds__(kP2GThreads, kCtasPerSm)
     k_batch_p2g(const SceneArgs<R>* __restrict__ A, const int32_t* __restrict__ start, int ns) {
     VB vb;
     const SceneArgs<R>& a = A[scene_of_block(start, ns, vb)];
-    p2g_body<R>(vb, a.sc, a.in, a.aux, a.bin, reinterpret_cast<R*>(a.grid.tile), a.cnt);
+    p2g_body(vb, a.sc, a.in, a.aux, a.bin, reinterpret_cast<R*>(a.grid.tile), a.cnt);
 }
 
-template <typename R>
-size_t p2g_smem_bytes() {
-    return p2g_stage_bytes<R>() + sizeof(P2GMeta<R>);
-}
+constexpr size_t kSmem = p2g_stage_bytes() + sizeof(P2GMeta);
 
-template <typename R>
-cudaError_t prepare_p2g() {
-    const int smem = (int)p2g_smem_bytes<R>();
-    cudaError_t e = cudaFuncSetAttribute(k_p2g<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch_p2g<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+}  // namespace
+
+template <>
+cudaError_t prepare_p2g<float>() {
+    cudaError_t e = cudaFuncSetAttribute(k_p2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch_p2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     return e;
 }
 
-template <typename R>
-int p2g_ctas(int nb_cap, int sms) {
-    return max(1, min(nb_cap, sms * p2g_ctas_per_sm<R>()));
+template <>
+int p2g_ctas<float>(int nb_cap, int sms) {
+    return max(1, min(nb_cap, sms * kCtasPerSm));
 }
-template int p2g_ctas<float>(int, int);
-template int p2g_ctas<double>(int, int);
 
-template <typename R>
-cudaError_t launch_batch_p2g(const SceneArgs<R>* A, const BatchPlan& P, cudaStream_t s) {
-    return launch_kernel(k_batch_p2g<R>, dim3((unsigned)P.total[BM_P2G]), dim3(kP2GThreads), p2g_smem_bytes<R>(), s, A,
-                         P.start[BM_P2G], P.n_scenes);
+template <>
+cudaError_t launch_batch_p2g<float>(const SceneArgs<float>* A, const BatchPlan& P, cudaStream_t s) {
+    return launch_kernel(k_batch_p2g, dim3((unsigned)P.total[BM_P2G]), dim3(kP2GThreads), kSmem, s, A, P.start[BM_P2G],
+                         P.n_scenes);
 }
-template cudaError_t launch_batch_p2g<float>(const SceneArgs<float>*, const BatchPlan&, cudaStream_t);
-template cudaError_t launch_batch_p2g<double>(const SceneArgs<double>*, const BatchPlan&, cudaStream_t);
-template cudaError_t prepare_p2g<float>();
-template cudaError_t prepare_p2g<double>();
 
-template <typename R>
-cudaError_t launch_p2g(const SceneDev<R>* sc, const PState<R>& st, const PAux<R>& aux, BinDev bin, GridDev grid,
-                       Counters* cnt, LaunchCfg cfg, cudaStream_t stream) {
-    k_p2g<R><<<p2g_ctas<R>(bin.nb_cap, cfg.num_sms), kP2GThreads, p2g_smem_bytes<R>(), stream>>>(
-        sc, st, aux, bin, reinterpret_cast<R*>(grid.tile), cnt);
+template <>
+cudaError_t launch_p2g<float>(const SceneDev<float>* sc, const PState<float>& st, const PAux<float>& aux, BinDev bin,
+                               GridDev grid, Counters* cnt, LaunchCfg cfg, cudaStream_t stream) {
+    k_p2g<<<p2g_ctas<float>(bin.nb_cap, cfg.num_sms), kP2GThreads, kSmem, stream>>>(
+        sc, st, aux, bin, reinterpret_cast<float*>(grid.tile), cnt);
     return cudaGetLastError();
 }
-
-template cudaError_t launch_p2g<float>(const SceneDev<float>*, const PState<float>&, const PAux<float>&, BinDev,
-                                       GridDev, Counters*, LaunchCfg, cudaStream_t);
-template cudaError_t launch_p2g<double>(const SceneDev<double>*, const PState<double>&, const PAux<double>&, BinDev,
-                                        GridDev, Counters*, LaunchCfg, cudaStream_t);
 
 }  // namespace gmpm
