@@ -269,6 +269,7 @@ struct Scene : SceneBase {
     // positions (set by a key pass or by the G2P that wrote them), so the next
     // binning skips its key pass
     bool keys_fresh = false;
+    bool grid_dirty = false;  // the last binning was batched and left its grid flags set
     int64_t launches = 0;  // kernels launched by this scene
     uint64_t uid_ = g_scene_uid++;
     int share_ = 0;        // SMs the launch shapes are sized for (0: all)
@@ -444,11 +445,11 @@ struct Scene : SceneBase {
             // a provisional pass with tiny capacities only to count pages
             bin.nb_cap = 1;
             bin.ng_cap = 1;
-            const int64_t scan_n = key_space;
-            scan.capacity = scan_scratch_elems(scan_n);
-            int32_t* ts = nullptr;
-            GMPM_TRY(alloc(&ts, (size_t)scan.capacity));
-            scan.tile_sums = ts;
+            uint32_t* words = nullptr;
+            GMPM_TRY(alloc(&words, (size_t)scan_scratch_words(key_space, 64)));
+            scan = scan_scratch(words, key_space, 64);
+            GMPM_TRY(alloc(&bin.block_keys, 1));
+            GMPM_TRY(alloc(&bin.grid_keys, 1));
             GMPM_TRY(count_pages(&nb0, &ng0));
         }
         int64_t nb_cap = desc.block_capacity > 0 ? desc.block_capacity : std::max<int64_t>(2 * (int64_t)nb0, nb0 + 256);
@@ -466,11 +467,15 @@ struct Scene : SceneBase {
         GMPM_TRY(alloc(&bin.adj, (size_t)nb_cap * 8));
         GMPM_TRY(alloc(&bin.grid_src, (size_t)ng_cap * 8));
         {
-            const int64_t scan_n = std::max<int64_t>(key_space, nb_cap * 64);
-            scan.capacity = scan_scratch_elems(scan_n);
-            int32_t* ts = nullptr;
-            GMPM_TRY(alloc(&ts, (size_t)scan.capacity));
-            scan.tile_sums = ts;
+            uint32_t* words = nullptr;
+            GMPM_TRY(alloc(&words, (size_t)scan_scratch_words(key_space, nb_cap * 64)));
+            int32_t* sums = nullptr;  // of the batched scans
+            GMPM_TRY(alloc(&sums, (size_t)scan_tiles(std::max<int64_t>(key_space, nb_cap * 64)) + 1));
+            scan = scan_scratch(words, key_space, nb_cap * 64, sums);
+            // zero between binnings (kernels.h)
+            GMPM_TRY(cudaMemset(scan.words, 0, (size_t)scan.count * sizeof(uint32_t)));
+            GMPM_TRY(cudaMemset(bin.cell_count, 0, (size_t)nb_cap * 64 * sizeof(int32_t)));
+            GMPM_TRY(cudaMemset(bin.grid_flag, 0, key_space));
         }
         R* tile = nullptr;
         R* nodes = nullptr;
@@ -506,15 +511,11 @@ struct Scene : SceneBase {
 
     // Count active and grid pages of the current positions (creation only).
     cudaError_t count_pages(int* nb, int* ng) {
-        const int T = 256;
-        const unsigned gk = (bin.key_space + T - 1) / T;
         cudaMemset(bin.page_flag, 0, bin.key_space);
         cudaMemset(bin.grid_flag, 0, bin.key_space);
+        cudaMemset(scan.words, 0, (size_t)scan.count * sizeof(uint32_t));
         launch_keys_only(0);
-        scan_exclusive<uint8_t>(bin.page_flag, bin.page_rank, (int64_t)bin.key_space, &d_cnt->n_blocks, scan, 0);
-        mark_grid(0);
-        scan_exclusive<uint8_t>(bin.grid_flag, bin.grid_rank, (int64_t)bin.key_space, &d_cnt->n_grid_blocks, scan, 0);
-        (void)gk;
+        launch_page_scans(bin, scan, d_cnt, 0);
         Counters h{};
         cudaError_t e = cudaMemcpy(&h, d_cnt, sizeof(h), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return e;
@@ -523,7 +524,6 @@ struct Scene : SceneBase {
         return cudaGetLastError();
     }
     void launch_keys_only(cudaStream_t s);
-    void mark_grid(cudaStream_t s);
 
     // A key pass over the current positions: keys and page flags.
     cudaError_t refresh_keys(cudaStream_t s) {
@@ -541,7 +541,8 @@ struct Scene : SceneBase {
     }
 
     gmpm_status do_bin(cudaStream_t s) {
-        GMPM_TRY(launch_binning<R>(d_sc, st[cur], bin, scan, d_cnt, cfg().num_sms, s));
+        GMPM_TRY(launch_binning<R>(d_sc, st[cur], bin, scan, d_cnt, cfg().num_sms, s, false, grid_dirty));
+        grid_dirty = false;
         binned = true;
         keys_fresh = true;
         return GMPM_OK;
@@ -557,7 +558,7 @@ struct Scene : SceneBase {
         const bool keys_ready = keys_fresh;
         keys_fresh = false;  // until this substep's G2P has keyed the new positions
         int64_t nk = (keys_ready ? kBinningKernelsKeysReady : kBinningKernels) + 4;
-        GMPM_TRY(launch_binning<R>(d_sc, st[c], bin, scan, d_cnt, lc.num_sms, s, keys_ready));
+        GMPM_TRY(launch_binning<R>(d_sc, st[c], bin, scan, d_cnt, lc.num_sms, s, keys_ready, grid_dirty));
         if (ev) GMPM_TRY(cudaEventRecord(ev[0], s));
         GMPM_TRY(launch_p2g<R>(d_sc, st[c], aux, bin, grid, d_cnt, lc, s));
         if (ev) GMPM_TRY(cudaEventRecord(ev[1], s));
@@ -591,6 +592,7 @@ struct Scene : SceneBase {
         gmpm_status r = launch_one(s, cur, ev, true, &nk);
         if (r != GMPM_OK) return r;
         commit_substeps(1);
+        grid_dirty = false;
         launches += nk - kernels_per_substep();
         return GMPM_OK;
     }
@@ -614,6 +616,7 @@ struct Scene : SceneBase {
         if (own_launches) launches += (int64_t)nsub * kernels_per_substep();  // as launched by a captured substep
         if (nsub & 1) cur = 1 - cur;
         binned = false;
+        grid_dirty = true;  // unless one_substep says otherwise
     }
     void set_sm_share(int sms) override { share_ = sms > 0 ? sms : 0; }
     int sm_share() const override { return share_; }
@@ -1026,10 +1029,6 @@ namespace gmpm {
 template <typename R>
 void Scene<R>::launch_keys_only(cudaStream_t s) {
     launch_keys<R>(d_sc, st[cur], bin, d_cnt, s);
-}
-template <typename R>
-void Scene<R>::mark_grid(cudaStream_t s) {
-    launch_mark_grid(bin, s);
 }
 }  // namespace gmpm
 

@@ -69,38 +69,118 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_keys(int64_t n, const R* __
     bin_keys_body<R>(own_blocks(), n, x0, x1, x2, sc, keys, page_flag, cnt);
 }
 
-// Mark every active page and its 7 "+" neighbours as grid pages
-// (supplementAdjacentPages, Transformer_kernal.cu:70-96).
-__device__ __forceinline__ void mark_grid_body(VB vb, uint32_t key_space, const uint8_t* __restrict__ page_flag,
-                                               uint8_t* __restrict__ grid_flag) {
-    const uint32_t k = vb.b * blockDim.x + threadIdx.x;
-    if (k >= key_space || !page_flag[k]) return;
-    int bx, by, bz;
-    page_coords(k, bx, by, bz);
+// Ranks of the flagged keys in ascending order, with their list and count:
+// page ids (the first scan) or grid page ids (the second).  The first also
+// marks every active page and its 7 "+" neighbours as grid pages
+// (supplementAdjacentPages, Transformer_kernal.cu:70-96).  words: the scan's
+// status words and, after them, its ticket.  Ranks of keys without a flag are
+// left as they are; no reader looks at them.
+__device__ __forceinline__ void page_scan_body(uint32_t key_space, const uint8_t* __restrict__ flag,
+                                               int32_t* __restrict__ rank, uint32_t* __restrict__ list, int cap,
+                                               int32_t* __restrict__ total, uint8_t* __restrict__ grid_flag,
+                                               uint32_t* __restrict__ words, Counters* cnt) {
+    const int ntiles = (int)((key_space + kScanTile - 1) / kScanTile);
+    const int tile = scan_take_tile(words + ntiles);
+    if (tile >= ntiles) return;
+    static_assert(kScanItems == 16, "one 16-byte load per thread");
+    const uint32_t k0 = (uint32_t)tile * kScanTile + threadIdx.x * kScanItems;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (k0 < key_space) v = *reinterpret_cast<const uint4*>(flag + k0);  // the key space is a multiple of 64
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t bits = 0;
 #pragma unroll
-    for (int d = 0; d < 8; ++d) grid_flag[page_key(bx + (d >> 2), by + ((d >> 1) & 1), bz + (d & 1))] = 1;
+    for (int q = 0; q < 4; ++q) bits |= ((w[q] | w[q] >> 7 | w[q] >> 14 | w[q] >> 21) & 15u) << (4 * q);
+    __shared__ int32_t tot;
+    int32_t run = block_exclusive_sum(__popc(bits), &tot);
+    bool bad;
+    const int32_t before = scan_look_back(words, tile, tot, bad);
+    run += before;
+    bool over = false;
+    while (bits) {
+        const uint32_t k = k0 + (uint32_t)__ffs((int)bits) - 1;
+        bits &= bits - 1;
+        rank[k] = run;
+        if (run < cap)
+            list[run] = k;
+        else
+            over = true;
+        ++run;
+        if (grid_flag) {
+            int bx, by, bz;
+            page_coords(k, bx, by, bz);
+#pragma unroll
+            for (int d = 0; d < 8; ++d) grid_flag[page_key(bx + (d >> 2), by + ((d >> 1) & 1), bz + (d & 1))] = 1;
+        }
+    }
+    if (over) raise_flag(cnt, GMPM_FLAG_TABLE_OVERFLOW);
+    if (tile == ntiles - 1 && threadIdx.x == 0) {
+        *total = bad ? 0 : before + tot;  // without a count nothing downstream runs
+        if (bad) raise_flag(cnt, GMPM_FLAG_COPY_TIMEOUT);
+    }
 }
 
-__global__ void k_mark_grid(uint32_t key_space, const uint8_t* __restrict__ page_flag, uint8_t* __restrict__ grid_flag) {
-    mark_grid_body(own_blocks(), key_space, page_flag, grid_flag);
+__global__ void __launch_bounds__(kScanThreads)
+    k_page_scan(uint32_t key_space, const uint8_t* __restrict__ flag, int32_t* __restrict__ rank,
+                uint32_t* __restrict__ list, int cap, int32_t* __restrict__ total, uint8_t* __restrict__ grid_flag,
+                uint32_t* __restrict__ words, Counters* cnt) {
+    page_scan_body(key_space, flag, rank, list, cap, total, grid_flag, words, cnt);
 }
 
-// Compact flagged keys into ascending order.
-__device__ __forceinline__ void compact_keys_body(VB vb, uint32_t key_space, const uint8_t* __restrict__ flag,
-                                                  const int32_t* __restrict__ rank, uint32_t* __restrict__ out,
-                                                  int cap, Counters* cnt) {
-    const uint32_t k = vb.b * blockDim.x + threadIdx.x;
-    if (k >= key_space || !flag[k]) return;
-    const int r = rank[k];
-    if (r < cap)
-        out[r] = k;
-    else
-        raise_flag(cnt, GMPM_FLAG_TABLE_OVERFLOW);
+// Zero `bytes` (a multiple of 16, from a 16-byte boundary) in 4 KiB pieces: pieces vb.b, vb.b + vb.g, ...
+__device__ __forceinline__ void zero_bytes_body(VB vb, void* p, int64_t bytes) {
+    char* c = static_cast<char*>(p);
+    for (int64_t off = (int64_t)vb.b * 4096 + (int64_t)threadIdx.x * 16; off < bytes; off += (int64_t)vb.g * 4096)
+        *reinterpret_cast<uint4*>(c + off) = make_uint4(0u, 0u, 0u, 0u);
 }
 
-__global__ void k_compact_keys(uint32_t key_space, const uint8_t* __restrict__ flag, const int32_t* __restrict__ rank,
-                               uint32_t* __restrict__ out, int cap, Counters* cnt) {
-    compact_keys_body(own_blocks(), key_space, flag, rank, out, cap, cnt);
+// Cell starts of the active pages (live cells; the capacity is larger) and the
+// total after them.  The starts also replace the counts, as the scatter's fill
+// pointers.  clear: flags whose last use in the binning was the page links,
+// cleared here for the next one (or null).
+__device__ __forceinline__ void cell_scan_body(VB vb, int64_t ncell, int32_t* __restrict__ count,
+                                               int32_t* __restrict__ start, uint32_t* __restrict__ words,
+                                               uint8_t* clear0, uint8_t* clear1, uint32_t key_space, Counters* cnt) {
+    if (clear0) zero_bytes_body(vb, clear0, key_space);
+    if (clear1) zero_bytes_body(vb, clear1, key_space);
+    const int64_t m = min(ncell, (int64_t)max(cnt->n_blocks, 0) * 64);
+    const int tile = scan_take_tile(words + (ncell + kScanTile - 1) / kScanTile);
+    const int64_t base = (int64_t)tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
+    if ((int64_t)tile * kScanTile >= max(m, (int64_t)1)) return;  // whole CTA; tile 0 writes the total of no cells
+    int4 v[kScanItems / 4];
+    int32_t s = 0;
+#pragma unroll
+    for (int q = 0; q < kScanItems / 4; ++q) {
+        // live cells come in pages of 64
+        v[q] = base + 4 * q < m ? *reinterpret_cast<const int4*>(count + base + 4 * q) : make_int4(0, 0, 0, 0);
+        s += v[q].x + v[q].y + v[q].z + v[q].w;
+    }
+    __shared__ int32_t tot;
+    int32_t run = block_exclusive_sum(s, &tot);
+    bool bad;
+    const int32_t before = scan_look_back(words, tile, tot, bad);
+    run += before;
+#pragma unroll
+    for (int q = 0; q < kScanItems / 4; ++q) {
+        const int4 o = make_int4(run, run + v[q].x, run + v[q].x + v[q].y, run + v[q].x + v[q].y + v[q].z);
+        if (base + 4 * q < m) {
+            *reinterpret_cast<int4*>(start + base + 4 * q) = o;
+            *reinterpret_cast<int4*>(count + base + 4 * q) = o;
+        }
+        run = o.w + v[q].w;
+    }
+    if (threadIdx.x == 0 && m <= (int64_t)(tile + 1) * kScanTile) {  // the tile of the last live cell
+        start[m] = before + tot;
+        if (bad) {
+            cnt->n_blocks = 0;
+            raise_flag(cnt, GMPM_FLAG_COPY_TIMEOUT);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+    k_cell_scan(int64_t ncell, int32_t* __restrict__ count, int32_t* __restrict__ start, uint32_t* __restrict__ words,
+                uint8_t* clear0, uint8_t* clear1, uint32_t key_space, Counters* cnt) {
+    cell_scan_body(own_blocks(), ncell, count, start, words, clear0, clear1, key_space, cnt);
 }
 
 // Page topology: adj (establishPageTopology, Transformer_kernal.cu:98-114) and
@@ -116,7 +196,7 @@ __device__ __forceinline__ void page_links_body(VB vb, const BinDev& bin, const 
         int bx, by, bz;
         page_coords(bin.block_keys[idx], bx, by, bz);
         const int r = bin.grid_rank[page_key(bx + di, by + dj, bz + dk)];
-        bin.adj[idx * 8 + slot] = (r < bin.ng_cap) ? r : -1;  // overflow is flagged by k_compact_keys
+        bin.adj[idx * 8 + slot] = (r < bin.ng_cap) ? r : -1;  // overflow is flagged by the page scan
     }
     if (idx < ng) {
         int gx, gy, gz;
@@ -132,8 +212,6 @@ __device__ __forceinline__ void page_links_body(VB vb, const BinDev& bin, const 
         bin.grid_src[idx * 8 + slot] = src;
     }
 }
-
-__global__ void k_page_links(BinDev bin, const Counters* cnt) { page_links_body(own_blocks(), bin, cnt); }
 
 // Histogram of (page rank, cell) buckets with warp-aggregated atomics.
 __device__ __forceinline__ void bin_hist_body(VB vb, int64_t n, const uint32_t* __restrict__ keys,
@@ -156,13 +234,27 @@ __device__ __forceinline__ void bin_hist_body(VB vb, int64_t n, const uint32_t* 
     }
 }
 
-__global__ void __launch_bounds__(kBinThreads) k_bin_hist(int64_t n, const uint32_t* __restrict__ keys,
-                                                          const int32_t* __restrict__ page_rank,
-                                                          int32_t* __restrict__ cell_count, int nb_cap) {
-    bin_hist_body(own_blocks(), n, keys, page_rank, cell_count, nb_cap);
+__host__ __device__ inline int bin_ctas(int64_t n) {
+    const int64_t c = (n + (int64_t)kBinThreads * kBinILP - 1) / ((int64_t)kBinThreads * kBinILP);
+    return c < 1 ? 1 : (int)c;
 }
 
-// Scatter slots; lanes of one warp with the same bucket keep their order.
+// The histogram's CTAs and, after them, the page links' (both need the ranks only).
+__device__ __forceinline__ void hist_links_body(VB vb, const BinDev& bin, const Counters* cnt) {
+    const int hist = bin_ctas(bin.n);
+    if (vb.b < hist)
+        bin_hist_body(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap);
+    else
+        page_links_body(VB{vb.b - hist, vb.g - hist}, bin, cnt);
+}
+
+__global__ void __launch_bounds__(kBinThreads) k_bin_hist_links(BinDev bin, const Counters* cnt) {
+    hist_links_body(own_blocks(), bin, cnt);
+}
+
+// Scatter slots; lanes of one warp with the same bucket keep their order.  fill: the cells' fill pointers, or
+// (kOffsets) fill counts beside the cells' starts.
+template <bool kOffsets>
 __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_t* __restrict__ keys,
                                                  const int32_t* __restrict__ page_rank,
                                                  const int32_t* __restrict__ cell_start, int32_t* __restrict__ fill,
@@ -179,7 +271,7 @@ __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_
         bucket[u] = r < nb_cap ? r * 64 + (int)(key[u] & 63) : -1;
     }
 #pragma unroll
-    for (int u = 0; u < kBinILP; ++u) start[u] = bucket[u] >= 0 ? cell_start[bucket[u]] : 0;
+    for (int u = 0; u < kBinILP; ++u) start[u] = kOffsets && bucket[u] >= 0 ? cell_start[bucket[u]] : 0;
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int u = 0; u < kBinILP; ++u) {
@@ -196,12 +288,9 @@ __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_
     }
 }
 
-__global__ void __launch_bounds__(kBinThreads) k_bin_scatter(int64_t n, const uint32_t* __restrict__ keys,
-                                                             const int32_t* __restrict__ page_rank,
-                                                             const int32_t* __restrict__ cell_start,
-                                                             int32_t* __restrict__ fill, int32_t* __restrict__ perm,
-                                                             uint32_t* __restrict__ keys_sorted, int nb_cap) {
-    bin_scatter_body(own_blocks(), n, keys, page_rank, cell_start, fill, perm, keys_sorted, nb_cap);
+__global__ void __launch_bounds__(kBinThreads) k_bin_scatter(BinDev bin) {
+    bin_scatter_body<false>(own_blocks(), bin.n, bin.keys, bin.page_rank, nullptr, bin.cell_count, bin.perm,
+                            bin.keys_sorted, bin.nb_cap);
 }
 
 // Canonical in-cell order: ascending previous slot.  Each warp takes one page
@@ -254,7 +343,8 @@ __device__ __forceinline__ void canon_rank_warp(const BinDev& bin, const int32_t
     }
 }
 
-__device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, Counters* cnt) {
+// Also clears, for the next binning, the fill pointers of the pages' cells and the scans' words.
+__device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, const ScanScratch& scan, Counters* cnt) {
     __shared__ int32_t buf[kCanonBuf];
     __shared__ int32_t cs[kCanonWarps][68];
     __shared__ uint8_t bad[kCanonWarps][64];
@@ -262,11 +352,14 @@ __device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, Counter
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = min(cnt->n_blocks, bin.nb_cap);
     int32_t* wbuf = buf + warp * kCanonWarpBuf;
+    if (vb.b == 0)
+        for (int q = threadIdx.x; q < scan.count; q += blockDim.x) scan.words[q] = 0u;
     for (int g = vb.b * kCanonWarps; g < nb; g += vb.g * kCanonWarps) {
         const int b = g + warp;
         int is_big = 0;
         if (b < nb) {
             for (int q = lane; q < 65; q += 32) cs[warp][q] = bin.cell_start[(int64_t)b * 64 + q];
+            for (int q = lane; q < 64; q += 32) bin.cell_count[(int64_t)b * 64 + q] = 0;
             __syncwarp();
             const int lo = cs[warp][0], hi = cs[warp][64];
             if (hi - lo <= kCanonWarpBuf) {
@@ -304,69 +397,73 @@ __device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, Counter
     }
 }
 
-__global__ void __launch_bounds__(32 * kCanonWarps) k_bin_canon(BinDev bin, Counters* cnt) {
-    bin_canon_body(own_blocks(), bin, cnt);
+__global__ void __launch_bounds__(32 * kCanonWarps) k_bin_canon(BinDev bin, ScanScratch scan, Counters* cnt) {
+    bin_canon_body(own_blocks(), bin, scan, cnt);
 }
+
+static int canon_ctas(int nb_cap, int sms) { return std::max(1, std::min((nb_cap + kCanonWarps - 1) / kCanonWarps, sms * 8)); }
 
 // ---------------------------------------------------------------------------
 
-static unsigned bin_grid(int64_t n) {
-    return (unsigned)std::max<int64_t>(1, (n + (int64_t)kBinThreads * kBinILP - 1) / ((int64_t)kBinThreads * kBinILP));
+static int links_ctas(const BinDev& bin) { return (int)(((int64_t)std::max(bin.nb_cap, bin.ng_cap) * 8 + 255) / 256); }
+
+static cudaError_t launch_page_scan(const BinDev& bin, const ScanScratch& scan, Counters* cnt, bool mark, cudaStream_t s) {
+    return launch_kernel(k_page_scan, dim3((unsigned)scan_tiles(bin.key_space)), dim3(kScanThreads), 0, s, bin.key_space,
+                         (const uint8_t*)bin.page_flag, bin.page_rank, bin.block_keys, (int)bin.nb_cap, &cnt->n_blocks,
+                         mark ? bin.grid_flag : nullptr, scan.words, cnt);
+}
+static cudaError_t launch_grid_scan(const BinDev& bin, const ScanScratch& scan, Counters* cnt, cudaStream_t s) {
+    return launch_kernel(k_page_scan, dim3((unsigned)scan_tiles(bin.key_space)), dim3(kScanThreads), 0, s, bin.key_space,
+                         (const uint8_t*)bin.grid_flag, bin.grid_rank, bin.grid_keys, (int)bin.ng_cap,
+                         &cnt->n_grid_blocks, (uint8_t*)nullptr, scan.words + scan.grid, cnt);
 }
 
-cudaError_t launch_bin_hist(int64_t n, const uint32_t* keys, const int32_t* page_rank, int32_t* cell_count, int nb_cap,
-                            cudaStream_t s) {
-    return launch_kernel(k_bin_hist, dim3(bin_grid(n)), dim3(kBinThreads), 0, s, n, keys, page_rank, cell_count,
-                         nb_cap);
+cudaError_t launch_page_scans(BinDev bin, ScanScratch scan, Counters* cnt, cudaStream_t s) {
+    const cudaError_t e = launch_page_scan(bin, scan, cnt, true, s);
+    return e == cudaSuccess ? launch_grid_scan(bin, scan, cnt, s) : e;
 }
 
-cudaError_t launch_bin_scatter(int64_t n, const uint32_t* keys, const int32_t* page_rank, const int32_t* cell_start,
-                               int32_t* fill, int32_t* perm, uint32_t* keys_sorted, int nb_cap, cudaStream_t s) {
-    return launch_kernel(k_bin_scatter, dim3(bin_grid(n)), dim3(kBinThreads), 0, s, n, keys, page_rank, cell_start,
-                         fill, perm, keys_sorted, nb_cap);
+// Histogram (with the page links where the binning has grid pages), cell scan, scatter, canonical order.
+static cudaError_t launch_bin_sort(const BinDev& bin, const ScanScratch& scan, Counters* cnt, int num_sms, bool clear_pages,
+                                   cudaStream_t s) {
+    const int64_t ncell = (int64_t)bin.nb_cap * 64;
+    const unsigned hist = (unsigned)(bin_ctas(bin.n) + (bin.grid_flag ? links_ctas(bin) : 0));
+    cudaError_t e = launch_kernel(k_bin_hist_links, dim3(hist), dim3(kBinThreads), 0, s, bin, (const Counters*)cnt);
+    if (e == cudaSuccess)
+        e = launch_kernel(k_cell_scan, dim3((unsigned)scan_tiles(ncell)), dim3(kScanThreads), 0, s, ncell, bin.cell_count,
+                          bin.cell_start, scan.words + scan.cells, clear_pages ? bin.page_flag : nullptr, bin.grid_flag,
+                          bin.key_space, cnt);
+    if (e == cudaSuccess)
+        e = launch_kernel(k_bin_scatter, dim3((unsigned)bin_ctas(bin.n)), dim3(kBinThreads), 0, s, bin);
+    if (e == cudaSuccess)
+        e = launch_kernel(k_bin_canon, dim3((unsigned)canon_ctas(bin.nb_cap, num_sms)), dim3(32 * kCanonWarps), 0, s, bin,
+                          scan, cnt);
+    return e;
 }
 
-cudaError_t launch_bin_canon(BinDev bin, Counters* cnt, int num_sms, cudaStream_t s) {
-    return launch_kernel(k_bin_canon, dim3(num_sms * 8), dim3(32 * kCanonWarps), 0, s, bin, cnt);
+cudaError_t launch_bin_no_grid(BinDev bin, ScanScratch scan, Counters* cnt, int num_sms, cudaStream_t s) {
+    const cudaError_t e = launch_page_scan(bin, scan, cnt, false, s);
+    return e == cudaSuccess ? launch_bin_sort(bin, scan, cnt, num_sms, true, s) : e;
 }
 
 template <typename R>
 cudaError_t launch_binning(const SceneDev<R>* sc, const PState<R>& st, BinDev bin, ScanScratch scan, Counters* cnt,
-                           int num_sms, cudaStream_t stream, bool keys_ready) {
-    const int64_t n = bin.n;
-    const int T = 256;
-    const unsigned gn = bin_grid(n);
-    const unsigned gk = (bin.key_space + T - 1) / T;
-    cudaMemsetAsync(bin.grid_flag, 0, bin.key_space, stream);
+                           int num_sms, cudaStream_t stream, bool keys_ready, bool clear_grid) {
+    if (clear_grid) cudaMemsetAsync(bin.grid_flag, 0, bin.key_space, stream);
     if (!keys_ready) {
         cudaMemsetAsync(bin.page_flag, 0, bin.key_space, stream);
-        k_bin_keys<R><<<gn, kBinThreads, 0, stream>>>(n, st.x[0], st.x[1], st.x[2], sc, bin.keys, bin.page_flag, cnt);
+        k_bin_keys<R><<<bin_ctas(bin.n), kBinThreads, 0, stream>>>(bin.n, st.x[0], st.x[1], st.x[2], sc, bin.keys,
+                                                                   bin.page_flag, cnt);
     }
-    scan_exclusive<uint8_t>(bin.page_flag, bin.page_rank, (int64_t)bin.key_space, &cnt->n_blocks, scan, stream);
-    k_mark_grid<<<gk, T, 0, stream>>>(bin.key_space, bin.page_flag, bin.grid_flag);
-    scan_exclusive<uint8_t>(bin.grid_flag, bin.grid_rank, (int64_t)bin.key_space, &cnt->n_grid_blocks, scan, stream);
-    k_compact_keys<<<gk, T, 0, stream>>>(bin.key_space, bin.page_flag, bin.page_rank, bin.block_keys, bin.nb_cap, cnt);
-    k_compact_keys<<<gk, T, 0, stream>>>(bin.key_space, bin.grid_flag, bin.grid_rank, bin.grid_keys, bin.ng_cap, cnt);
-    const int links = max(bin.nb_cap, bin.ng_cap) * 8;
-    k_page_links<<<(links + T - 1) / T, T, 0, stream>>>(bin, cnt);
-    // the page flags' last use was the links: cleared for the G2P that keys the next positions
-    if (keys_ready) cudaMemsetAsync(bin.page_flag, 0, bin.key_space, stream);
-    const int64_t ncell = (int64_t)bin.nb_cap * 64;
-    cudaMemsetAsync(bin.cell_count, 0, ncell * sizeof(int32_t), stream);
-    launch_bin_hist(n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap, stream);
-    // the cells of the active pages only (the page scan above counted them)
-    scan_exclusive<int32_t>(bin.cell_count, bin.cell_start, ncell, bin.cell_start + ncell, scan, stream,
-                            &cnt->n_blocks);
-    cudaMemsetAsync(bin.cell_count, 0, ncell * sizeof(int32_t), stream);
-    launch_bin_scatter(n, bin.keys, bin.page_rank, bin.cell_start, bin.cell_count, bin.perm, bin.keys_sorted,
-                       bin.nb_cap, stream);
-    launch_bin_canon(bin, cnt, num_sms, stream);
-    return cudaGetLastError();
+    cudaError_t e = launch_page_scans(bin, scan, cnt, stream);
+    // with keys_ready the page flags are cleared after their last use, for the G2P that keys the next positions
+    if (e == cudaSuccess) e = launch_bin_sort(bin, scan, cnt, num_sms, keys_ready, stream);
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 template <typename R>
 cudaError_t launch_keys(const SceneDev<R>* sc, const PState<R>& st, BinDev bin, Counters* cnt, cudaStream_t s) {
-    k_bin_keys<R><<<bin_grid(bin.n), kBinThreads, 0, s>>>(bin.n, st.x[0], st.x[1], st.x[2], sc, bin.keys,
+    k_bin_keys<R><<<bin_ctas(bin.n), kBinThreads, 0, s>>>(bin.n, st.x[0], st.x[1], st.x[2], sc, bin.keys,
                                                                  bin.page_flag, cnt);
     return cudaGetLastError();
 }
@@ -375,12 +472,6 @@ template cudaError_t launch_keys<float>(const SceneDev<float>*, const PState<flo
 template cudaError_t launch_keys<double>(const SceneDev<double>*, const PState<double>&, BinDev, Counters*,
                                          cudaStream_t);
 
-cudaError_t launch_mark_grid(BinDev bin, cudaStream_t s) {
-    const int T = 256;
-    k_mark_grid<<<(bin.key_space + T - 1) / T, T, 0, s>>>(bin.key_space, bin.page_flag, bin.grid_flag);
-    return cudaGetLastError();
-}
-
 // ---- batched binning over many scenes ------------------------------------------
 
 void batch_scene_ctas(int64_t n, uint32_t key_space, int nb_cap, int ng_cap, int sms, int real_bytes,
@@ -388,13 +479,13 @@ void batch_scene_ctas(int64_t n, uint32_t key_space, int nb_cap, int ng_cap, int
     auto cdiv = [](int64_t a, int64_t b) { return (int)std::max<int64_t>(1, (a + b - 1) / b); };
     const int64_t ncell = (int64_t)nb_cap * 64;
     ctas[BM_ZERO_FLAGS] = cdiv(key_space, 4096);
-    ctas[BM_PARTICLES] = (int)bin_grid(n);
+    ctas[BM_PARTICLES] = bin_ctas(n);
     ctas[BM_KEYSPACE] = cdiv(key_space, 256);
-    ctas[BM_KEY_TILES] = cdiv(key_space, kScanTile);
+    ctas[BM_KEY_TILES] = (int)scan_tiles(key_space);
     ctas[BM_LINKS] = cdiv((int64_t)std::max(nb_cap, ng_cap) * 8, 256);
     ctas[BM_ZERO_CELLS] = cdiv(ncell * 4, 4096);
-    ctas[BM_CELL_TILES] = cdiv(ncell, kScanTile);
-    ctas[BM_CANON] = std::max(1, std::min(cdiv(nb_cap, kCanonWarps), sms * 8));
+    ctas[BM_CELL_TILES] = (int)scan_tiles(ncell);
+    ctas[BM_CANON] = canon_ctas(nb_cap, sms);
     ctas[BM_P2G] = real_bytes == 4 ? p2g_ctas<float>(nb_cap, sms) : p2g_ctas<double>(nb_cap, sms);
     ctas[BM_GRID] = std::max(1, std::min(ng_cap / 4 + 1, sms * 8));
     const int per_sm = real_bytes == 4 ? 2 : 1;  // G2P's resident CTAs per SM
@@ -402,19 +493,29 @@ void batch_scene_ctas(int64_t n, uint32_t key_space, int nb_cap, int ng_cap, int
     ctas[BM_ONE] = 1;
 }
 
-// Zero `bytes` (a multiple of 4) from p in 4 KiB pieces: pieces vb.b, vb.b + vb.g, ...
-__device__ __forceinline__ void zero_bytes_body(VB vb, void* p, int64_t bytes) {
-    char* c = static_cast<char*>(p);
-    const bool aligned = (reinterpret_cast<uintptr_t>(c) & 15) == 0;
-    for (int64_t piece = (int64_t)vb.b * 4096; piece < bytes; piece += (int64_t)vb.g * 4096) {
-        const int64_t off = piece + (int64_t)threadIdx.x * 16;
-        if (off + 16 <= bytes && aligned) {
-            *reinterpret_cast<uint4*>(c + off) = make_uint4(0u, 0u, 0u, 0u);
-        } else {
-            for (int q = 0; q < 16; q += 4)
-                if (off + q + 4 <= bytes) *reinterpret_cast<uint32_t*>(c + off + q) = 0u;
-        }
-    }
+// Mark every active page and its 7 "+" neighbours as grid pages
+// (supplementAdjacentPages, Transformer_kernal.cu:70-96).
+__device__ __forceinline__ void mark_grid_body(VB vb, uint32_t key_space, const uint8_t* __restrict__ page_flag,
+                                               uint8_t* __restrict__ grid_flag) {
+    const uint32_t k = vb.b * blockDim.x + threadIdx.x;
+    if (k >= key_space || !page_flag[k]) return;
+    int bx, by, bz;
+    page_coords(k, bx, by, bz);
+#pragma unroll
+    for (int d = 0; d < 8; ++d) grid_flag[page_key(bx + (d >> 2), by + ((d >> 1) & 1), bz + (d & 1))] = 1;
+}
+
+// Compact flagged keys into ascending order.
+__device__ __forceinline__ void compact_keys_body(VB vb, uint32_t key_space, const uint8_t* __restrict__ flag,
+                                                  const int32_t* __restrict__ rank, uint32_t* __restrict__ out,
+                                                  int cap, Counters* cnt) {
+    const uint32_t k = vb.b * blockDim.x + threadIdx.x;
+    if (k >= key_space || !flag[k]) return;
+    const int r = rank[k];
+    if (r < cap)
+        out[r] = k;
+    else
+        raise_flag(cnt, GMPM_FLAG_TABLE_OVERFLOW);
 }
 
 // which: 1 grid flags; 2 cell counters; 3 cell counters and page flags (after
@@ -527,7 +628,7 @@ __global__ void __launch_bounds__(kBinThreads) k_batch_scatter(const SceneArgs<R
                                                                const int32_t* __restrict__ start, int ns) {
     VB vb;
     const BinDev& bin = A[scene_of_block(start, ns, vb)].bin;
-    bin_scatter_body(vb, bin.n, bin.keys, bin.page_rank, bin.cell_start, bin.cell_count, bin.perm, bin.keys_sorted,
+    bin_scatter_body<true>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_start, bin.cell_count, bin.perm, bin.keys_sorted,
                      bin.nb_cap);
 }
 
@@ -536,11 +637,11 @@ __global__ void __launch_bounds__(32 * kCanonWarps) k_batch_canon(const SceneArg
                                                                   const int32_t* __restrict__ start, int ns) {
     VB vb;
     const SceneArgs<R>& a = A[scene_of_block(start, ns, vb)];
-    bin_canon_body(vb, a.bin, a.cnt);
+    bin_canon_body(vb, a.bin, a.scan, a.cnt);
 }
 
 // The binning of every scene of a batch: the same steps as launch_binning with
-// keys_ready, each one launch over all scenes.
+// keys_ready, each one launch over all scenes, with the scans in three passes.
 template <typename R>
 cudaError_t launch_batch_binning(const SceneArgs<R>* A, const BatchPlan& P, cudaStream_t s) {
     const int ns = P.n_scenes;
@@ -570,8 +671,8 @@ template cudaError_t launch_batch_binning<float>(const SceneArgs<float>*, const 
 template cudaError_t launch_batch_binning<double>(const SceneArgs<double>*, const BatchPlan&, cudaStream_t);
 
 template cudaError_t launch_binning<float>(const SceneDev<float>*, const PState<float>&, BinDev, ScanScratch,
-                                           Counters*, int, cudaStream_t, bool);
+                                           Counters*, int, cudaStream_t, bool, bool);
 template cudaError_t launch_binning<double>(const SceneDev<double>*, const PState<double>&, BinDev, ScanScratch,
-                                            Counters*, int, cudaStream_t, bool);
+                                            Counters*, int, cudaStream_t, bool, bool);
 
 }  // namespace gmpm

@@ -55,23 +55,20 @@ struct LaunchCfg {
 // st's positions (written by the G2P that produced them), so the key pass is
 // skipped and the page flags are cleared after their last use, for the next
 // G2P to set.  Otherwise the key pass runs and the flags stay set.
+// clear_grid: a batched binning left its grid flags set.
 template <typename R>
 cudaError_t launch_binning(const SceneDev<R>* sc, const PState<R>& st, BinDev bin, ScanScratch scan, Counters* cnt,
-                           int num_sms, cudaStream_t stream, bool keys_ready = false);
+                           int num_sms, cudaStream_t stream, bool keys_ready = false, bool clear_grid = false);
 // Kernels launched by launch_binning without / with keys_ready.
-constexpr int kBinningKernels = 17;
-constexpr int kBinningKernelsKeysReady = 16;
+constexpr int kBinningKernels = 7;
+constexpr int kBinningKernelsKeysReady = 6;
 
-// Keys + page flags only, and grid-page marking (used to size capacities).
+// Keys + page flags only, and the page and grid page scans (used to size capacities).
 template <typename R>
 cudaError_t launch_keys(const SceneDev<R>* sc, const PState<R>& st, BinDev bin, Counters* cnt, cudaStream_t s);
-cudaError_t launch_mark_grid(BinDev bin, cudaStream_t s);
-// The counting-sort passes of the binning (also used by the allocation-free entry point).
-cudaError_t launch_bin_hist(int64_t n, const uint32_t* keys, const int32_t* page_rank, int32_t* cell_count, int nb_cap,
-                            cudaStream_t s);
-cudaError_t launch_bin_scatter(int64_t n, const uint32_t* keys, const int32_t* page_rank, const int32_t* cell_start,
-                               int32_t* fill, int32_t* perm, uint32_t* keys_sorted, int nb_cap, cudaStream_t s);
-cudaError_t launch_bin_canon(BinDev bin, Counters* cnt, int num_sms, cudaStream_t s);
+cudaError_t launch_page_scans(BinDev bin, ScanScratch scan, Counters* cnt, cudaStream_t s);
+// The binning without grid pages (the allocation-free entry point): keys and page flags are set, bin.grid_flag is null.
+cudaError_t launch_bin_no_grid(BinDev bin, ScanScratch scan, Counters* cnt, int num_sms, cudaStream_t s);
 
 // Number of components of a gmpm_field (0 if unknown).
 int field_components(int field);
@@ -173,7 +170,7 @@ __device__ __forceinline__ const SceneArgs<R>& batch_scene_args(const SceneArgs<
 // Per-scene CTA ranges of the stages (device arrays of n_scenes + 1 starts).
 enum BatchMap : int {
     BM_ZERO_FLAGS = 0,  // key_space bytes in 4 KiB pieces
-    BM_PARTICLES,       // particles, 4 per thread (histogram, scatter)
+    BM_PARTICLES,       // particles, 8 per thread (histogram, scatter)
     BM_KEYSPACE,        // one thread per page key (grid marking, compaction)
     BM_KEY_TILES,       // scan tiles of the key space
     BM_LINKS,           // page links

@@ -43,15 +43,13 @@ constexpr size_t kOffBlockKeys = align256(kOffPageRank + kNoAllocKeySpace * size
 constexpr size_t kOffCellCount = align256(kOffBlockKeys + kNoAllocKeySpace * sizeof(uint32_t));
 constexpr size_t kOffCellStart = align256(kOffCellCount + kNoAllocCells * sizeof(int32_t));
 constexpr size_t kOffScanTiles = align256(kOffCellStart + (kNoAllocCells + 1) * sizeof(int32_t));
-constexpr size_t kScanTilesElems = (kNoAllocCells + kScanTile - 1) / kScanTile + 1;
-constexpr size_t kNoAllocScratchBytes = align256(kOffScanTiles + kScanTilesElems * sizeof(int32_t));
+// status words of the page scan, an unused grid scan and the cell scan, with their tickets
+constexpr size_t kScanWords =
+    2 * ((kNoAllocKeySpace + kScanTile - 1) / kScanTile + 1) + (kNoAllocCells + kScanTile - 1) / kScanTile + 1;
+constexpr size_t kNoAllocScratchBytes = align256(kOffScanTiles + kScanWords * sizeof(uint32_t));
 static_assert(kNoAllocScratchBytes == GMPM_NOALLOC_SCRATCH_BYTES, "keep include/gmpm.h in step");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
-
-// Kernel of bin.cu reused unchanged (the counting-sort passes go through the launchers of kernels.h).
-__global__ void k_compact_keys(uint32_t key_space, const uint8_t* __restrict__ flag, const int32_t* __restrict__ rank,
-                               uint32_t* __restrict__ out, int cap, Counters* cnt);
 
 // Page/cell keys of interleaved xyz positions: the scene binning's cell_key
 // (common.cuh; cal_cellId, Particle_kernal.cu:158-165).
@@ -124,7 +122,7 @@ extern "C" gmpm_status gmpm_bin_positions_noalloc(const float* positions, int64_
     bin.block_keys = reinterpret_cast<uint32_t*>(base + kOffBlockKeys);
     bin.cell_count = reinterpret_cast<int32_t*>(base + kOffCellCount);
     bin.cell_start = reinterpret_cast<int32_t*>(base + kOffCellStart);
-    ScanScratch scan{reinterpret_cast<int32_t*>(base + kOffScanTiles), (int64_t)kScanTilesElems};
+    const ScanScratch scan = scan_scratch(reinterpret_cast<uint32_t*>(base + kOffScanTiles), kNoAllocKeySpace, ncell);
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -133,26 +131,13 @@ extern "C" gmpm_status gmpm_bin_positions_noalloc(const float* positions, int64_
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(Counters), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(bin.page_flag, 0, kNoAllocKeySpace, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(bin.cell_count, 0, ncell * sizeof(int32_t), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(scan.words, 0, scan.count * sizeof(uint32_t), s);
     const int T = 256;
     const unsigned gn = (unsigned)((n + T - 1) / T);
-    const unsigned gk = (kNoAllocKeySpace + T - 1) / T;
     if (e == cudaSuccess)
         e = launch_kernel(k_noalloc_keys, dim3(gn), dim3(T), 0, s, n, positions, 1.0 / dx, res_x, res_y, res_z,
                           bin.keys, bin.page_flag, cnt);
-    if (e == cudaSuccess)
-        e = scan_exclusive<uint8_t>(bin.page_flag, bin.page_rank, (int64_t)kNoAllocKeySpace, &cnt->n_blocks, scan, s);
-    if (e == cudaSuccess)
-        e = launch_kernel(k_compact_keys, dim3(gk), dim3(T), 0, s, kNoAllocKeySpace, (const uint8_t*)bin.page_flag,
-                          (const int32_t*)bin.page_rank, bin.block_keys, (int)bin.nb_cap, cnt);
-    if (e == cudaSuccess) e = launch_bin_hist(n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap, s);
-    if (e == cudaSuccess)
-        e = scan_exclusive<int32_t>(bin.cell_count, bin.cell_start, ncell, bin.cell_start + ncell, scan, s,
-                                    &cnt->n_blocks);
-    if (e == cudaSuccess) e = cudaMemsetAsync(bin.cell_count, 0, ncell * sizeof(int32_t), s);
-    if (e == cudaSuccess)
-        e = launch_bin_scatter(n, bin.keys, bin.page_rank, bin.cell_start, bin.cell_count, perm, keys_sorted,
-                               bin.nb_cap, s);
-    if (e == cudaSuccess) e = launch_bin_canon(bin, cnt, sms, s);
+    if (e == cudaSuccess) e = launch_bin_no_grid(bin, scan, cnt, sms, s);
     if (e == cudaSuccess && flags)
         e = cudaMemcpyAsync(flags, &cnt->flags, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? GMPM_OOM : GMPM_CUDA_ERROR;

@@ -1,6 +1,13 @@
-// Device-wide exclusive prefix sum (reduce -> scan tile sums -> apply), used
-// for page ranks and cell offsets.  Replaces the reference's recursive block
-// scan and Thrust scans (cuda_kernal_tools.cu:15-203, Transformer_kernal.cu:142-207).
+// Device-wide exclusive prefix sums of the binning: page ranks and cell starts.
+// Replaces the reference's recursive block scan and Thrust scans
+// (cuda_kernal_tools.cu:15-203, Transformer_kernal.cu:142-207).
+//
+// One pass ("decoupled look-back", Merrill and Garland, "Single-pass Parallel
+// Prefix Scan with Decoupled Look-back", 2016): a CTA takes the next tile from
+// a ticket, sums it, and gets the sum of the tiles before it from their status
+// words.  Tiles are taken in order, so every tile waited for is held by a CTA
+// that already runs.  A batch, whose launches serve all its scenes, scans in
+// three passes (tile sums, their scan, apply: the bodies at the end).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -14,18 +21,23 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-struct ScanScratch {
-    int32_t* tile_sums;  // capacity: ceil(max_n / kScanTile) + 1
-    int64_t capacity;
-};
+inline int64_t scan_tiles(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
 
-template <typename TIn>
-__device__ __forceinline__ void scan_load(const TIn* in, int64_t n, int64_t base, int32_t v[kScanItems]) {
-#pragma unroll
-    for (int q = 0; q < kScanItems; ++q) {
-        const int64_t idx = base + q;
-        v[q] = (idx < n) ? (int32_t)in[idx] : 0;
-    }
+// Working words of the binning's three scans (page flags, grid flags, cell
+// counts), one after the other: a status word per tile and the ticket.  They
+// are zero between binnings (the last kernel of a binning clears them).
+struct ScanScratch {
+    uint32_t* words;
+    int32_t count;
+    int32_t grid, cells;  // first word of the second and the third scan
+    int32_t* tile_sums;   // the batched scans' tile sums: one per tile of the longer of the key space and the cells, + 1
+};
+inline int64_t scan_scratch_words(int64_t key_space, int64_t ncell) {
+    return 2 * (scan_tiles(key_space) + 1) + scan_tiles(ncell) + 1;
+}
+inline ScanScratch scan_scratch(uint32_t* words, int64_t key_space, int64_t ncell, int32_t* tile_sums = nullptr) {
+    const int32_t k = (int32_t)scan_tiles(key_space) + 1;
+    return ScanScratch{words, (int32_t)scan_scratch_words(key_space, ncell), k, 2 * k, tile_sums};
 }
 
 __device__ __forceinline__ int32_t block_exclusive_sum(int32_t x, int32_t* total) {
@@ -56,6 +68,73 @@ __device__ __forceinline__ int32_t block_exclusive_sum(int32_t x, int32_t* total
     return r;
 }
 
+// Status word of a tile: its own sum, or the sum up to and with it; both bits:
+// a wait gave up.  Sums stay below 2^28 (the particle limit).
+enum : uint32_t { kScanSum = 1u << 30, kScanPrefix = 2u << 30, kScanBad = 3u << 30, kScanValue = (1u << 30) - 1 };
+constexpr int kScanSpinLimit = 1 << 22;
+
+// The CTA's next tile.
+__device__ __forceinline__ int scan_take_tile(uint32_t* ticket) {
+    __shared__ int s_tile;
+    if (threadIdx.x == 0) s_tile = (int)atomicAdd(ticket, 1u);
+    __syncthreads();
+    return s_tile;
+}
+
+// Sum of the tiles before `tile`, whose own sum is `total`; every thread of the
+// CTA calls it.  `bad`: a wait gave up here or before (the sum is then 0).
+__device__ __forceinline__ int32_t scan_look_back(uint32_t* status, int tile, int32_t total, bool& bad) {
+    __shared__ int32_t s_prefix;
+    __shared__ int s_bad;
+    volatile uint32_t* st = status;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int32_t prefix = 0;
+        bool gave_up = false;
+        if (tile > 0) {
+            if (lane == 0) st[tile] = kScanSum | (uint32_t)total;
+            for (int end = tile - 1;; end -= 32) {
+                const int i = end - lane;
+                uint32_t s = i >= 0 ? st[i] : kScanPrefix;
+                for (int spin = 0; __any_sync(0xffffffffu, s == 0); ++spin) {
+                    if (spin >= kScanSpinLimit) {
+                        if (s == 0) s = kScanBad;
+                        break;
+                    }
+                    if (s == 0) s = st[i];
+                }
+                const unsigned ends = __ballot_sync(0xffffffffu, (s & kScanPrefix) != 0);
+                const int last = ends ? __ffs(ends) - 1 : 31;
+                if (__any_sync(0xffffffffu, lane <= last && s >= kScanBad)) {
+                    gave_up = true;
+                    break;
+                }
+                prefix += (int32_t)__reduce_add_sync(0xffffffffu, lane <= last ? (s & kScanValue) : 0u);
+                if (ends) break;
+            }
+        }
+        if (lane == 0) {
+            st[tile] = gave_up ? kScanBad : kScanPrefix | (uint32_t)(prefix + total);
+            s_prefix = gave_up ? 0 : prefix;
+            s_bad = gave_up;
+        }
+    }
+    __syncthreads();
+    bad = s_bad != 0;
+    return s_prefix;
+}
+
+// ---- three-pass scan of a batch (vb: the CTA's tile within its scene's scan) ---
+
+template <typename TIn>
+__device__ __forceinline__ void scan_load(const TIn* in, int64_t n, int64_t base, int32_t v[kScanItems]) {
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q) {
+        const int64_t idx = base + q;
+        v[q] = (idx < n) ? (int32_t)in[idx] : 0;
+    }
+}
+
 // Entries scanned: all n, or with `live` (a device count of live blocks of 64
 // entries, the active pages of a cell scan, whose capacity is larger) only the
 // live entries.  The scan then writes the live entries and the one after them,
@@ -65,8 +144,6 @@ __device__ __forceinline__ int64_t scan_live_len(int64_t n, const int32_t* live)
     return live ? min(n, (int64_t)max(*live, 0) * 64) : n;
 }
 
-// Bodies take the CTA's tile index within its scene's scan (VB, common.cuh),
-// so that the same code serves one-scene and batched launches.
 template <typename TIn>
 __device__ __forceinline__ void scan_reduce_body(VB vb, const TIn* __restrict__ in, int64_t n,
                                                  int32_t* __restrict__ tile_sums, const int32_t* live = nullptr) {
@@ -84,13 +161,6 @@ __device__ __forceinline__ void scan_reduce_body(VB vb, const TIn* __restrict__ 
     __shared__ int32_t tot;
     block_exclusive_sum(s, &tot);
     if (threadIdx.x == 0) tile_sums[vb.b] = tot;
-}
-
-template <typename TIn>
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const TIn* __restrict__ in, int64_t n,
-                                                               int32_t* __restrict__ tile_sums,
-                                                               const int32_t* __restrict__ live) {
-    scan_reduce_body(own_blocks(), in, n, tile_sums, live);
 }
 
 // Single CTA: exclusive scan of the tile sums in place, total to *total.
@@ -117,11 +187,6 @@ __device__ __forceinline__ void scan_tiles_body(int32_t* __restrict__ tile_sums,
     if (threadIdx.x == 0) *total = carry;
 }
 
-static __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(int32_t* __restrict__ tile_sums, int64_t ntiles,
-                                                              int32_t* __restrict__ total) {
-    scan_tiles_body(tile_sums, ntiles, total);
-}
-
 template <typename TIn>
 __device__ __forceinline__ void scan_apply_body(VB vb, const TIn* __restrict__ in, int64_t n,
                                                 const int32_t* __restrict__ tile_offsets, int32_t* __restrict__ out,
@@ -143,31 +208,5 @@ __device__ __forceinline__ void scan_apply_body(VB vb, const TIn* __restrict__ i
         run += v[q];
     }
 }
-
-template <typename TIn>
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const TIn* __restrict__ in, int64_t n,
-                                                              const int32_t* __restrict__ tile_offsets,
-                                                              int32_t* __restrict__ out,
-                                                              const int32_t* __restrict__ live) {
-    scan_apply_body(own_blocks(), in, n, tile_offsets, out, live);
-}
-
-// out[i] = sum_{j<i} in[j] for i < n; *total = sum of all.  With `live` (see
-// scan_live_len) only the live entries are read and the live entries and the
-// one after them written.  Returns the status of its own launches.
-template <typename TIn>
-inline cudaError_t scan_exclusive(const TIn* in, int32_t* out, int64_t n, int32_t* total, ScanScratch s,
-                                  cudaStream_t stream, const int32_t* live = nullptr) {
-    const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    cudaError_t e = launch_kernel(k_scan_reduce<TIn>, dim3((unsigned)ntiles), dim3(kScanThreads), 0, stream, in, n,
-                                  s.tile_sums, live);
-    if (e == cudaSuccess) e = launch_kernel(k_scan_tiles, dim3(1), dim3(kScanThreads), 0, stream, s.tile_sums, ntiles, total);
-    if (e == cudaSuccess)
-        e = launch_kernel(k_scan_apply<TIn>, dim3((unsigned)ntiles), dim3(kScanThreads), 0, stream, in, n,
-                          (const int32_t*)s.tile_sums, out, live);
-    return e;
-}
-
-inline int64_t scan_scratch_elems(int64_t max_n) { return (max_n + kScanTile - 1) / kScanTile + 1; }
 
 }  // namespace gmpm

@@ -58,11 +58,11 @@ struct BinDev {
     uint32_t* keys_sorted;  // [n] sorted keys
     int32_t* perm;          // [n] new slot -> previous slot
     uint8_t* page_flag;     // [key_space]
-    int32_t* page_rank;     // [key_space] exclusive scan of page_flag
-    uint8_t* grid_flag;     // [key_space]
+    int32_t* page_rank;     // [key_space] rank of each flagged page
+    uint8_t* grid_flag;     // [key_space] zero between binnings, except after a batched one
     int32_t* grid_rank;     // [key_space]
     uint32_t* block_keys;   // [nb_cap]
-    int32_t* cell_count;    // [nb_cap*64] histogram, then scatter fill counters
+    int32_t* cell_count;    // [nb_cap*64] histogram, then scatter fill pointers; zero between binnings
     int32_t* cell_start;    // [nb_cap*64 + 1]
     uint32_t* grid_keys;    // [ng_cap]
     int32_t* adj;           // [nb_cap*8]  grid index of page + (i,j,k), slot 4i+2j+k
