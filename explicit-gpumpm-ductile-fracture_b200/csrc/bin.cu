@@ -22,6 +22,12 @@ namespace gmpm {
 // their loads before using any, so more requests are in flight per SM.
 constexpr int kBinThreads = 256;
 constexpr int kBinILP = 8;
+// Scenes that would leave SMs without a CTA take two particles per thread: the
+// scatter's chain of loads and atomics is then latency, not throughput (131k
+// particles: histogram and scatter 5 and 10 us at eight per thread).
+constexpr int kBinSmallILP = 2;
+constexpr int64_t kBinSmall = (int64_t)2 * 148 * kBinThreads * kBinILP;
+__host__ __device__ inline int bin_ilp(int64_t n) { return n < kBinSmall ? kBinSmallILP : kBinILP; }
 
 // The kernels' bodies take the CTA's index within its scene's share of the
 // launch (VB, common.cuh); the __global__ wrappers below each body serve a
@@ -214,67 +220,66 @@ __device__ __forceinline__ void page_links_body(VB vb, const BinDev& bin, const 
 }
 
 // Histogram of (page rank, cell) buckets with warp-aggregated atomics.
+template <int kILP>
 __device__ __forceinline__ void bin_hist_body(VB vb, int64_t n, const uint32_t* __restrict__ keys,
                                               const int32_t* __restrict__ page_rank, int32_t* __restrict__ cell_count,
                                               int nb_cap) {
-    const int64_t i0 = (int64_t)vb.b * kBinThreads * kBinILP + threadIdx.x;
-    uint32_t key[kBinILP];
-    int rank[kBinILP];
+    const int64_t i0 = (int64_t)vb.b * kBinThreads * kILP + threadIdx.x;
+    uint32_t key[kILP];
+    int rank[kILP];
 #pragma unroll
-    for (int u = 0; u < kBinILP; ++u) key[u] = i0 + (int64_t)u * kBinThreads < n ? keys[i0 + (int64_t)u * kBinThreads] : 0u;
+    for (int u = 0; u < kILP; ++u) key[u] = i0 + (int64_t)u * kBinThreads < n ? keys[i0 + (int64_t)u * kBinThreads] : 0u;
 #pragma unroll
-    for (int u = 0; u < kBinILP; ++u)
+    for (int u = 0; u < kILP; ++u)
         rank[u] = i0 + (int64_t)u * kBinThreads < n ? page_rank[key[u] >> 6] : nb_cap;
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int u = 0; u < kBinILP; ++u) {
+    for (int u = 0; u < kILP; ++u) {
         const int bucket = rank[u] < nb_cap ? rank[u] * 64 + (int)(key[u] & 63) : -1;
         const unsigned peers = __match_any_sync(0xffffffffu, bucket);
         if (bucket >= 0 && lane == __ffs(peers) - 1) atomicAdd(&cell_count[bucket], __popc(peers));
     }
 }
 
-__host__ __device__ inline int bin_ctas(int64_t n) {
-    const int64_t c = (n + (int64_t)kBinThreads * kBinILP - 1) / ((int64_t)kBinThreads * kBinILP);
+__host__ __device__ inline int bin_ctas(int64_t n, int ilp) {
+    const int64_t c = (n + (int64_t)kBinThreads * ilp - 1) / ((int64_t)kBinThreads * ilp);
     return c < 1 ? 1 : (int)c;
 }
 
 // The histogram's CTAs and, after them, the page links' (both need the ranks only).
-__device__ __forceinline__ void hist_links_body(VB vb, const BinDev& bin, const Counters* cnt) {
-    const int hist = bin_ctas(bin.n);
+template <int kILP>
+__global__ void __launch_bounds__(kBinThreads) k_bin_hist_links(BinDev bin, const Counters* cnt) {
+    const VB vb = own_blocks();
+    const int hist = bin_ctas(bin.n, kILP);
     if (vb.b < hist)
-        bin_hist_body(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap);
+        bin_hist_body<kILP>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap);
     else
         page_links_body(VB{vb.b - hist, vb.g - hist}, bin, cnt);
 }
 
-__global__ void __launch_bounds__(kBinThreads) k_bin_hist_links(BinDev bin, const Counters* cnt) {
-    hist_links_body(own_blocks(), bin, cnt);
-}
-
 // Scatter slots; lanes of one warp with the same bucket keep their order.  fill: the cells' fill pointers, or
 // (kOffsets) fill counts beside the cells' starts.
-template <bool kOffsets>
+template <int kILP, bool kOffsets>
 __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_t* __restrict__ keys,
                                                  const int32_t* __restrict__ page_rank,
                                                  const int32_t* __restrict__ cell_start, int32_t* __restrict__ fill,
                                                  int32_t* __restrict__ perm, uint32_t* __restrict__ keys_sorted,
                                                  int nb_cap) {
-    const int64_t i0 = (int64_t)vb.b * kBinThreads * kBinILP + threadIdx.x;
-    uint32_t key[kBinILP];
-    int bucket[kBinILP], start[kBinILP];
+    const int64_t i0 = (int64_t)vb.b * kBinThreads * kILP + threadIdx.x;
+    uint32_t key[kILP];
+    int bucket[kILP], start[kILP];
 #pragma unroll
-    for (int u = 0; u < kBinILP; ++u) key[u] = i0 + (int64_t)u * kBinThreads < n ? keys[i0 + (int64_t)u * kBinThreads] : 0u;
+    for (int u = 0; u < kILP; ++u) key[u] = i0 + (int64_t)u * kBinThreads < n ? keys[i0 + (int64_t)u * kBinThreads] : 0u;
 #pragma unroll
-    for (int u = 0; u < kBinILP; ++u) {
+    for (int u = 0; u < kILP; ++u) {
         const int r = i0 + (int64_t)u * kBinThreads < n ? page_rank[key[u] >> 6] : nb_cap;
         bucket[u] = r < nb_cap ? r * 64 + (int)(key[u] & 63) : -1;
     }
 #pragma unroll
-    for (int u = 0; u < kBinILP; ++u) start[u] = kOffsets && bucket[u] >= 0 ? cell_start[bucket[u]] : 0;
+    for (int u = 0; u < kILP; ++u) start[u] = kOffsets && bucket[u] >= 0 ? cell_start[bucket[u]] : 0;
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int u = 0; u < kBinILP; ++u) {
+    for (int u = 0; u < kILP; ++u) {
         const unsigned peers = __match_any_sync(0xffffffffu, bucket[u]);
         const int leader = __ffs(peers) - 1;
         int base = 0;
@@ -288,9 +293,10 @@ __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_
     }
 }
 
+template <int kILP>
 __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(BinDev bin) {
-    bin_scatter_body<false>(own_blocks(), bin.n, bin.keys, bin.page_rank, nullptr, bin.cell_count, bin.perm,
-                            bin.keys_sorted, bin.nb_cap);
+    bin_scatter_body<kILP, false>(own_blocks(), bin.n, bin.keys, bin.page_rank, nullptr, bin.cell_count, bin.perm,
+                                  bin.keys_sorted, bin.nb_cap);
 }
 
 // Canonical in-cell order: ascending previous slot.  Each warp takes one page
@@ -320,20 +326,41 @@ __device__ __forceinline__ void canon_rank(const BinDev& bin, const int32_t* cs,
     }
 }
 
+// The cell of slot s (cs: the page's 65 cell starts).
+__device__ __forceinline__ int cell_of_slot(const int32_t* cs, int s) {
+    int c = 0;  // the last cell that starts at or before s and is not empty there
+#pragma unroll
+    for (int step = 32; step > 0; step >>= 1)
+        if (cs[c + step] <= s) c += step;
+    return c;
+}
+
 // Warp path: the scatter keeps the order of the lanes of one warp, so most
-// cells already ascend by previous slot.  Only the cells with a descent are
-// ranked; an ascending cell is its own canonical order.
+// cells already ascend by previous slot; an ascending cell is its own canonical
+// order.  desc: a bit per slot that descends from the one before, less the
+// first slots of cells.  Only where one is left are the cells looked up and
+// the descending ones ranked.
 __device__ __forceinline__ void canon_rank_warp(const BinDev& bin, const int32_t* cs, const int32_t* buf,
-                                                uint8_t* bad, int lo, int hi, int lane) {
-    for (int c = lane; c < 64; c += 32) bad[c] = 0;
-    __syncwarp();
-    for (int s = lo + lane; s < hi; s += 32) {
-        const int cell = (int)(bin.keys_sorted[s] & 63);
-        if (s > cs[cell] && buf[s - lo - 1] > buf[s - lo]) bad[cell] = 1;
+                                                uint32_t* desc, uint8_t* bad, int lo, int hi, int lane) {
+    const int n = hi - lo, words = (n + 31) >> 5;
+    for (int w = 0; w < words; ++w) {
+        const int s = 32 * w + lane;
+        const unsigned d = __ballot_sync(0xffffffffu, s > 0 && s < n && buf[s - 1] > buf[s]);
+        if (lane == 0) desc[w] = d;
     }
     __syncwarp();
+    for (int c = lane; c < 64; c += 32) {
+        const int s = cs[c] - lo;
+        if (s < n) atomicAnd(&desc[s >> 5], ~(1u << (s & 31)));
+        bad[c] = 0;
+    }
+    __syncwarp();
+    const uint32_t mine = lane < words ? desc[lane] : 0u;
+    if (!__any_sync(0xffffffffu, mine != 0u)) return;
+    for (uint32_t d = mine; d; d &= d - 1) bad[cell_of_slot(cs, lo + 32 * lane + __ffs((int)d) - 1)] = 1;
+    __syncwarp();
     for (int s = lo + lane; s < hi; s += 32) {
-        const int cell = (int)(bin.keys_sorted[s] & 63);
+        const int cell = cell_of_slot(cs, s);
         if (!bad[cell]) continue;
         const int a = cs[cell] - lo, e = cs[cell + 1] - lo;
         const int32_t v = buf[s - lo];
@@ -348,6 +375,8 @@ __device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, const S
     __shared__ int32_t buf[kCanonBuf];
     __shared__ int32_t cs[kCanonWarps][68];
     __shared__ uint8_t bad[kCanonWarps][64];
+    __shared__ uint32_t desc[kCanonWarps][kCanonWarpBuf / 32];
+    static_assert(kCanonWarpBuf / 32 <= 32, "one word of slots per lane");
     __shared__ int big[kCanonWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = min(cnt->n_blocks, bin.nb_cap);
@@ -363,9 +392,17 @@ __device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, const S
             __syncwarp();
             const int lo = cs[warp][0], hi = cs[warp][64];
             if (hi - lo <= kCanonWarpBuf) {
-                for (int s = lo + lane; s < hi; s += 32) wbuf[s - lo] = bin.perm[s];
+                // eight loads in flight per lane: one at a time, a page was a chain of 12 round trips
+                for (int s0 = lo + lane; s0 < hi; s0 += 32 * 8) {
+                    int32_t v[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) v[u] = s0 + 32 * u < hi ? bin.perm[s0 + 32 * u] : 0;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (s0 + 32 * u < hi) wbuf[s0 + 32 * u - lo] = v[u];
+                }
                 __syncwarp();
-                canon_rank_warp(bin, cs[warp], wbuf, bad[warp], lo, hi, lane);
+                canon_rank_warp(bin, cs[warp], wbuf, desc[warp], bad[warp], lo, hi, lane);
             } else {
                 is_big = 1;
             }
@@ -427,14 +464,15 @@ cudaError_t launch_page_scans(BinDev bin, ScanScratch scan, Counters* cnt, cudaS
 static cudaError_t launch_bin_sort(const BinDev& bin, const ScanScratch& scan, Counters* cnt, int num_sms, bool clear_pages,
                                    cudaStream_t s) {
     const int64_t ncell = (int64_t)bin.nb_cap * 64;
-    const unsigned hist = (unsigned)(bin_ctas(bin.n) + (bin.grid_flag ? links_ctas(bin) : 0));
-    cudaError_t e = launch_kernel(k_bin_hist_links, dim3(hist), dim3(kBinThreads), 0, s, bin, (const Counters*)cnt);
+    const int ilp = bin_ilp(bin.n), ctas = bin_ctas(bin.n, ilp);
+    const unsigned hist = (unsigned)(ctas + (bin.grid_flag ? links_ctas(bin) : 0));
+    cudaError_t e = launch_kernel(ilp == kBinILP ? k_bin_hist_links<kBinILP> : k_bin_hist_links<kBinSmallILP>, dim3(hist), dim3(kBinThreads), 0, s, bin, (const Counters*)cnt);
     if (e == cudaSuccess)
         e = launch_kernel(k_cell_scan, dim3((unsigned)scan_tiles(ncell)), dim3(kScanThreads), 0, s, ncell, bin.cell_count,
                           bin.cell_start, scan.words + scan.cells, clear_pages ? bin.page_flag : nullptr, bin.grid_flag,
                           bin.key_space, cnt);
     if (e == cudaSuccess)
-        e = launch_kernel(k_bin_scatter, dim3((unsigned)bin_ctas(bin.n)), dim3(kBinThreads), 0, s, bin);
+        e = launch_kernel(ilp == kBinILP ? k_bin_scatter<kBinILP> : k_bin_scatter<kBinSmallILP>, dim3((unsigned)ctas), dim3(kBinThreads), 0, s, bin);
     if (e == cudaSuccess)
         e = launch_kernel(k_bin_canon, dim3((unsigned)canon_ctas(bin.nb_cap, num_sms)), dim3(32 * kCanonWarps), 0, s, bin,
                           scan, cnt);
@@ -452,7 +490,7 @@ cudaError_t launch_binning(const SceneDev<R>* sc, const PState<R>& st, BinDev bi
     if (clear_grid) cudaMemsetAsync(bin.grid_flag, 0, bin.key_space, stream);
     if (!keys_ready) {
         cudaMemsetAsync(bin.page_flag, 0, bin.key_space, stream);
-        k_bin_keys<R><<<bin_ctas(bin.n), kBinThreads, 0, stream>>>(bin.n, st.x[0], st.x[1], st.x[2], sc, bin.keys,
+        k_bin_keys<R><<<bin_ctas(bin.n, kBinILP), kBinThreads, 0, stream>>>(bin.n, st.x[0], st.x[1], st.x[2], sc, bin.keys,
                                                                    bin.page_flag, cnt);
     }
     cudaError_t e = launch_page_scans(bin, scan, cnt, stream);
@@ -463,7 +501,7 @@ cudaError_t launch_binning(const SceneDev<R>* sc, const PState<R>& st, BinDev bi
 
 template <typename R>
 cudaError_t launch_keys(const SceneDev<R>* sc, const PState<R>& st, BinDev bin, Counters* cnt, cudaStream_t s) {
-    k_bin_keys<R><<<bin_ctas(bin.n), kBinThreads, 0, s>>>(bin.n, st.x[0], st.x[1], st.x[2], sc, bin.keys,
+    k_bin_keys<R><<<bin_ctas(bin.n, kBinILP), kBinThreads, 0, s>>>(bin.n, st.x[0], st.x[1], st.x[2], sc, bin.keys,
                                                                  bin.page_flag, cnt);
     return cudaGetLastError();
 }
@@ -479,7 +517,7 @@ void batch_scene_ctas(int64_t n, uint32_t key_space, int nb_cap, int ng_cap, int
     auto cdiv = [](int64_t a, int64_t b) { return (int)std::max<int64_t>(1, (a + b - 1) / b); };
     const int64_t ncell = (int64_t)nb_cap * 64;
     ctas[BM_ZERO_FLAGS] = cdiv(key_space, 4096);
-    ctas[BM_PARTICLES] = bin_ctas(n);
+    ctas[BM_PARTICLES] = bin_ctas(n, kBinILP);
     ctas[BM_KEYSPACE] = cdiv(key_space, 256);
     ctas[BM_KEY_TILES] = (int)scan_tiles(key_space);
     ctas[BM_LINKS] = cdiv((int64_t)std::max(nb_cap, ng_cap) * 8, 256);
@@ -620,7 +658,7 @@ __global__ void __launch_bounds__(kBinThreads) k_batch_hist(const SceneArgs<R>* 
                                                             const int32_t* __restrict__ start, int ns) {
     VB vb;
     const BinDev& bin = A[scene_of_block(start, ns, vb)].bin;
-    bin_hist_body(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap);
+    bin_hist_body<kBinILP>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap);
 }
 
 template <typename R>
@@ -628,7 +666,7 @@ __global__ void __launch_bounds__(kBinThreads) k_batch_scatter(const SceneArgs<R
                                                                const int32_t* __restrict__ start, int ns) {
     VB vb;
     const BinDev& bin = A[scene_of_block(start, ns, vb)].bin;
-    bin_scatter_body<true>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_start, bin.cell_count, bin.perm, bin.keys_sorted,
+    bin_scatter_body<kBinILP, true>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_start, bin.cell_count, bin.perm, bin.keys_sorted,
                      bin.nb_cap);
 }
 
