@@ -339,7 +339,11 @@ __device__ __forceinline__ int cell_of_slot(const int32_t* cs, int s) {
 // cells already ascend by previous slot; an ascending cell is its own canonical
 // order.  desc: a bit per slot that descends from the one before, less the
 // first slots of cells.  Only where one is left are the cells looked up and
-// the descending ones ranked.
+// the descending ones ranked: a few of them one after the other, a lane per
+// particle, many (positions in no order) a lane per slot of the page (1M
+// shuffled positions: 164 us of binning against 177; sorted ones, 8.4M
+// particles: 150 against 140).
+constexpr int kCanonFewCells = 24;
 __device__ __forceinline__ void canon_rank_warp(const BinDev& bin, const int32_t* cs, const int32_t* buf,
                                                 uint32_t* desc, uint8_t* bad, int lo, int hi, int lane) {
     const int n = hi - lo, words = (n + 31) >> 5;
@@ -359,15 +363,31 @@ __device__ __forceinline__ void canon_rank_warp(const BinDev& bin, const int32_t
     if (!__any_sync(0xffffffffu, mine != 0u)) return;
     for (uint32_t d = mine; d; d &= d - 1) bad[cell_of_slot(cs, lo + 32 * lane + __ffs((int)d) - 1)] = 1;
     __syncwarp();
-    for (int s = lo + lane; s < hi; s += 32) {
-        const int cell = cell_of_slot(cs, s);
-        if (!bad[cell]) continue;
-        const int a = cs[cell] - lo, e = cs[cell + 1] - lo;
-        const int32_t v = buf[s - lo];
-        int r = 0;
-        for (int u = a; u < e; ++u) r += buf[u] < v;
-        bin.perm[lo + a + r] = v;
+    const unsigned b0 = __ballot_sync(0xffffffffu, bad[lane] != 0), b1 = __ballot_sync(0xffffffffu, bad[32 + lane] != 0);
+    if (__popc(b0) + __popc(b1) > kCanonFewCells) {
+        for (int s = lo + lane; s < hi; s += 32) {
+            const int cell = cell_of_slot(cs, s);
+            if (!bad[cell]) continue;
+            const int a = cs[cell] - lo, e = cs[cell + 1] - lo;
+            const int32_t v = buf[s - lo];
+            int r = 0;
+            for (int u = a; u < e; ++u) r += buf[u] < v;
+            bin.perm[lo + a + r] = v;
+        }
+        return;
     }
+#pragma unroll
+    for (int h = 0; h < 64; h += 32)
+        for (unsigned cells = h ? b1 : b0; cells; cells &= cells - 1) {
+            const int cell = h + __ffs((int)cells) - 1;
+            const int a = cs[cell] - lo, e = cs[cell + 1] - lo;
+            for (int s = a + lane; s < e; s += 32) {
+                const int32_t v = buf[s];
+                int r = 0;
+                for (int u = a; u < e; ++u) r += buf[u] < v;
+                bin.perm[lo + a + r] = v;
+            }
+        }
 }
 
 // Also clears, for the next binning, the fill pointers of the pages' cells and the scans' words.
