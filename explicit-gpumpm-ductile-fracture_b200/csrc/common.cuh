@@ -29,8 +29,11 @@ enum P2GChannel : int {
     kP2GChannels = 9
 };
 
-// Grid channels read by G2P.
+// Grid results read by G2P: per grid page the 64 nodes' (v0, v1, v2, dc) as one
+// word each, then the 64 nodes' c_new, so that a window copies a node with two
+// copies instead of five.
 enum GridChannel : int { GC_V0 = 0, GC_V1 = 1, GC_V2 = 2, GC_DC = 3, GC_CN = 4, kGridChannels = 5 };
+__host__ __device__ inline int grid_channel_at(int ch, int node) { return ch < 4 ? node * 4 + ch : 256 + node; }
 
 // Per-material constants in the precision of the kernel.
 template <typename Real>
@@ -138,8 +141,7 @@ __device__ inline void raise_flag(Counters* c, unsigned int f) { atomicOr(&c->fl
 // the grid is clamped to its edge and sets `bad`.  Shared by the binning's key
 // pass and G2P, which keys the positions it writes.
 template <typename R>
-__device__ __forceinline__ uint32_t cell_key(const R x[3], double inv_dx, const int res[3], bool& bad) {
-    int base[3];
+__device__ __forceinline__ void cell_base(const R x[3], double inv_dx, const int res[3], bool& bad, int base[3]) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int hi = res[a] - 3;
@@ -154,8 +156,15 @@ __device__ __forceinline__ uint32_t cell_key(const R x[3], double inv_dx, const 
             base[a] = (int)t - 1;
         }
     }
-    const uint32_t cell = (uint32_t)(((base[0] & 3) << 4) | ((base[1] & 3) << 2) | (base[2] & 3));
-    return (page_key(base[0] >> 2, base[1] >> 2, base[2] >> 2) << 6) | cell;
+}
+__device__ __forceinline__ uint32_t cell_of_base(const int base[3]) {
+    return (uint32_t)(((base[0] & 3) << 4) | ((base[1] & 3) << 2) | (base[2] & 3));
+}
+template <typename R>
+__device__ __forceinline__ uint32_t cell_key(const R x[3], double inv_dx, const int res[3], bool& bad) {
+    int base[3];
+    cell_base(x, inv_dx, res, bad, base);
+    return (page_key(base[0] >> 2, base[1] >> 2, base[2] >> 2) << 6) | cell_of_base(base);
 }
 
 // ---- launches over one scene or many ------------------------------------------

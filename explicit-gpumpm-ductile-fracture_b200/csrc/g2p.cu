@@ -61,10 +61,10 @@ struct G2PShared {
     uint32_t key[3][kG2PUnit];
     int32_t adj[kPageRing][8];
     uint32_t bkey[kPageRing];
+    int4 bpos[kPageRing];                // first node of the page (4 bx, 4 by, 4 bz) and its key, from bkey
     int32_t unit[3][UD_WORDS];
-    // per window value w = ch * 216 + node: source offset in its grid page
-    // (bits 0-8), neighbour slot (9-11), destination offset (12-21), c_new flag (22)
-    uint32_t wtab[kGridChannels * kWindowNodes];
+    // per window node: its node in its grid page (bits 0-5) and the neighbour slot of that page (6-8)
+    uint16_t wtab[kWindowNodes];
     // the cell-key parameters, read where each particle's key is formed (not
     // held in registers across the loop)
     double key_inv_dx;
@@ -361,6 +361,19 @@ __device__ __forceinline__ void issue_meta(G2PShared<R>& S, int m, int s0, int n
     }
 }
 
+// Page positions of a unit, whose meta has arrived.
+template <typename R>
+__device__ __forceinline__ void decode_pages(G2PShared<R>& S, int seq0, int np) {
+    const int t = threadIdx.x;
+    if (t < np) {
+        const int q = (seq0 + t) % kPageRing;
+        const uint32_t key = S.bkey[q];
+        int bx, by, bz;
+        page_coords(key, bx, by, bz);
+        S.bpos[q] = make_int4(4 * bx, 4 * by, 4 * bz, (int)key);
+    }
+}
+
 // Particle inputs of a unit, and the windows of its pages with sequence
 // numbers in [wseq0, wseq1) (the pages not staged by the previous unit).
 template <typename R>
@@ -380,15 +393,19 @@ __device__ __forceinline__ void issue_data(G2PShared<R>& S, int m, int buf, int 
     for (int wseq = wseq0; wseq < wseq1; ++wseq) {
         const int wbuf = wseq % kWinRing;
         const int32_t* adj = S.adj[wseq % kPageRing];
-        for (int w = t; w < kGridChannels * kWindowNodes; w += kG2PUnit) {
-            const uint32_t e = S.wtab[w];
-            const int g = adj[(e >> 9) & 7];
-            const int off = (int)((e >> 12) & 1023);
-            R* dst = (e >> 22) ? &S.wincn[wbuf][off] : &S.win4[wbuf][0][0] + off;
-            if (g >= 0)
-                cp_async_elem(dst, nodes + (int64_t)g * kGridChannels * 64 + (e & 511));
-            else
-                *dst = R(0);
+        // a thread per node: its word and its c_new
+        if (t < kWindowNodes) {
+            const uint32_t e = S.wtab[t];
+            const int g = adj[e >> 6];
+            const R* src = nodes + (int64_t)g * kGridChannels * 64;
+            Word4<R>* word = reinterpret_cast<Word4<R>*>(&S.win4[wbuf][t][0]);
+            if (g >= 0) {
+                cp_async_word(word, reinterpret_cast<const Word4<R>*>(src) + (e & 63));
+                cp_async_elem(&S.wincn[wbuf][t], src + grid_channel_at(GC_CN, (int)(e & 63)));
+            } else {
+                *word = Word4<R>{};
+                S.wincn[wbuf][t] = R(0);
+            }
         }
     }
 }
@@ -431,18 +448,15 @@ __device__ __forceinline__ void g2p_body(VB vb, const SceneDev<R>* __restrict__ 
     issue_meta(S, 0, d0[0], d0[1], d0[2], d0[3], d0[6], bin);
     cp_async_commit();
     // window copy table, once per CTA (the divisions of the node index)
-    for (int w = t; w < kGridChannels * kWindowNodes; w += kG2PUnit) {
-        const int ch = w / kWindowNodes;
-        const int node = w - ch * kWindowNodes;
-        const int a = node / 36, bb = (node / 6) % 6, cc = node % 6;
+    if (t < kWindowNodes) {
+        const int a = t / 36, bb = (t / 6) % 6, cc = t % 6;
         const int d = ((a >> 2) << 2) | ((bb >> 2) << 1) | (cc >> 2);
-        const uint32_t src = (uint32_t)(ch * 64 + (a & 3) * 16 + (bb & 3) * 4 + (cc & 3));
-        const uint32_t dst = (uint32_t)(ch < 4 ? node * 4 + ch : node);
-        S.wtab[w] = src | ((uint32_t)d << 9) | (dst << 12) | ((uint32_t)(ch == 4) << 22);
+        S.wtab[t] = (uint16_t)(((a & 3) * 16 + (bb & 3) * 4 + (cc & 3)) | (d << 6));
     }
     cp_async_wait_all();
     __syncthreads();
     int staged = d0[2] + d0[3];  // pages with sequence numbers below this have their window staged
+    if (d0[1] > 0) decode_pages(S, d0[2], d0[3]);
     issue_data(S, 0, 0, d0[1], d0[1] > 0 ? d0[2] : 0, d0[1] > 0 ? staged : 0, in, nodes);
     issue_meta(S, 1, d1[0], d1[1], d1[2], d1[3], d1[6], bin);
     cp_async_commit();
@@ -468,6 +482,7 @@ __device__ __forceinline__ void g2p_body(VB vb, const SceneDev<R>* __restrict__ 
                 w0 = max(u1seq, staged);
                 w1 = u1seq + u1np;
                 staged = max(staged, w1);
+                decode_pages(S, u1seq, u1np);
             }
             issue_data(S, m1, (k + 1) & 1, u1n, w0, w1, in, nodes);
             issue_meta(S, m2, d2[0], d2[1], d2[2], d2[3], d2[6], bin);
@@ -478,12 +493,11 @@ __device__ __forceinline__ void g2p_body(VB vb, const SceneDev<R>* __restrict__ 
             const int slot = u0s + t;
             // the particle's page within the unit
             const int pseq = u0seq + (u0np > 1 && slot >= u0c1) + (u0np > 2 && slot >= u0c2);
-            int bx, by, bz;
-            page_coords(S.bkey[pseq % kPageRing], bx, by, bz);
+            const int4 page = S.bpos[pseq % kPageRing];
             const uint32_t cell = S.key[m0][t] & 63u;
             const int li = (int)(cell >> 4), lj = (int)((cell >> 2) & 3), lk = (int)(cell & 3);
             const R x[3] = {S.p[buf][P_X][t], S.p[buf][P_X + 1][t], S.p[buf][P_X + 2][t]};
-            const R xp[3] = {x[0] - R(4 * bx + li) * dx, x[1] - R(4 * by + lj) * dx, x[2] - R(4 * bz + lk) * dx};
+            const R xp[3] = {x[0] - R(page.x + li) * dx, x[1] - R(page.y + lj) * dx, x[2] - R(page.z + lk) * dx};
             R wx[3], gx[3], wy[3], gy[3], wz[3], gz[3];
             bspline1d_g(xp[0], inv_dx, wx, gx);
             bspline1d_g(xp[1], inv_dx, wy, gy);
@@ -513,9 +527,17 @@ __device__ __forceinline__ void g2p_body(VB vb, const SceneDev<R>* __restrict__ 
                 // the new position's cell key and page, which the next
                 // substep's binning reads instead of running its key pass
                 bool bad = false;
-                const uint32_t key = cell_key(xn, S.key_inv_dx, S.key_res, bad);
+                int base[3];
+                cell_base(xn, S.key_inv_dx, S.key_res, bad, base);
+                // most particles stay in their page, whose key needs no interleaving again (the page is read
+                // again: held over the gather, its four words spill)
+                const volatile int4& pg = S.bpos[pseq % kPageRing];
+                uint32_t pkey = (uint32_t)pg.w;
+                if ((((base[0] ^ pg.x) | (base[1] ^ pg.y) | (base[2] ^ pg.z)) & ~3) != 0)
+                    pkey = page_key(base[0] >> 2, base[1] >> 2, base[2] >> 2);
+                const uint32_t key = (pkey << 6) | cell_of_base(base);
                 bin.keys[slot] = key;
-                bin.page_flag[key >> 6] = 1;
+                bin.page_flag[pkey] = 1;
                 if (bad) flags |= GMPM_FLAG_OUT_OF_DOMAIN;
             }
 #pragma unroll

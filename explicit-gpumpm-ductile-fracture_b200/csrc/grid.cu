@@ -128,9 +128,9 @@ __device__ __forceinline__ void grid_body(VB vb, const SceneDev<R>* __restrict__
             pcg.x[i] = pcg.r[i] = pcg.mr[i] = pcg.s[i] = pcg.q[i] = pcg.d[i] = pcg.cg[i] = 0.0;
             pcg.tag[i] = 0;
         }
-        R* N = nodes + (int64_t)g * kGridChannels * 64 + node;
-#pragma unroll
-        for (int q = 0; q < kGridChannels; ++q) N[q * 64] = out[q];
+        R* N = nodes + (int64_t)g * kGridChannels * 64;
+        *reinterpret_cast<Word4<R>*>(N + grid_channel_at(GC_V0, node)) = Word4<R>{{out[0], out[1], out[2], out[3]}};
+        N[grid_channel_at(GC_CN, node)] = out[GC_CN];
     }
     // FP64 conservation diagnostics of the P2G result
 #pragma unroll

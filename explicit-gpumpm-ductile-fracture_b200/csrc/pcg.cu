@@ -471,9 +471,10 @@ __global__ void k_pcg_finish(BinDev bin, PcgDev P, R* __restrict__ nodes, Counte
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         if (!P.tag[i]) continue;
         const double x = blow ? 1e20 : P.x[i];
-        R* nd = nodes + (int64_t)(i >> 6) * kGridChannels * 64 + (i & 63);
-        nd[GC_DC * 64] = (R)(x - P.cg[i]);
-        nd[GC_CN * 64] = (R)x;
+        R* nd = nodes + (int64_t)(i >> 6) * kGridChannels * 64;
+        const int node = (int)(i & 63);
+        nd[grid_channel_at(GC_DC, node)] = (R)(x - P.cg[i]);
+        nd[grid_channel_at(GC_CN, node)] = (R)x;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt->pcg_iterations = P.scal->iterations;
 }
