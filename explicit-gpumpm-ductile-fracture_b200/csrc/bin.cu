@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(kScanThreads)
     k_page_scan(uint32_t key_space, const uint8_t* __restrict__ flag, int32_t* __restrict__ rank,
                 uint32_t* __restrict__ list, int cap, int32_t* __restrict__ total, uint8_t* __restrict__ grid_flag,
                 uint32_t* __restrict__ words, Counters* cnt) {
+    depend_on_previous();
     page_scan_body(key_space, flag, rank, list, cap, total, grid_flag, words, cnt);
 }
 
@@ -186,6 +187,7 @@ __device__ __forceinline__ void cell_scan_body(VB vb, int64_t ncell, int32_t* __
 __global__ void __launch_bounds__(kScanThreads)
     k_cell_scan(int64_t ncell, int32_t* __restrict__ count, int32_t* __restrict__ start, uint32_t* __restrict__ words,
                 uint8_t* clear0, uint8_t* clear1, uint32_t key_space, Counters* cnt) {
+    depend_on_previous();
     cell_scan_body(own_blocks(), ncell, count, start, words, clear0, clear1, key_space, cnt);
 }
 
@@ -249,6 +251,7 @@ __host__ __device__ inline int bin_ctas(int64_t n, int ilp) {
 // The histogram's CTAs and, after them, the page links' (both need the ranks only).
 template <int kILP>
 __global__ void __launch_bounds__(kBinThreads) k_bin_hist_links(BinDev bin, const Counters* cnt) {
+    depend_on_previous();
     const VB vb = own_blocks();
     const int hist = bin_ctas(bin.n, kILP);
     if (vb.b < hist)
@@ -295,6 +298,7 @@ __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_
 
 template <int kILP>
 __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(BinDev bin) {
+    depend_on_previous();
     bin_scatter_body<kILP, false>(own_blocks(), bin.n, bin.keys, bin.page_rank, nullptr, bin.cell_count, bin.perm,
                                   bin.keys_sorted, bin.nb_cap);
 }
@@ -455,6 +459,7 @@ __device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, const S
 }
 
 __global__ void __launch_bounds__(32 * kCanonWarps) k_bin_canon(BinDev bin, ScanScratch scan, Counters* cnt) {
+    depend_on_previous();
     bin_canon_body(own_blocks(), bin, scan, cnt);
 }
 
@@ -465,12 +470,12 @@ static int canon_ctas(int nb_cap, int sms) { return std::max(1, std::min((nb_cap
 static int links_ctas(const BinDev& bin) { return (int)(((int64_t)std::max(bin.nb_cap, bin.ng_cap) * 8 + 255) / 256); }
 
 static cudaError_t launch_page_scan(const BinDev& bin, const ScanScratch& scan, Counters* cnt, bool mark, cudaStream_t s) {
-    return launch_kernel(k_page_scan, dim3((unsigned)scan_tiles(bin.key_space)), dim3(kScanThreads), 0, s, bin.key_space,
+    return launch_dependent(k_page_scan, dim3((unsigned)scan_tiles(bin.key_space)), dim3(kScanThreads), 0, s, bin.key_space,
                          (const uint8_t*)bin.page_flag, bin.page_rank, bin.block_keys, (int)bin.nb_cap, &cnt->n_blocks,
                          mark ? bin.grid_flag : nullptr, scan.words, cnt);
 }
 static cudaError_t launch_grid_scan(const BinDev& bin, const ScanScratch& scan, Counters* cnt, cudaStream_t s) {
-    return launch_kernel(k_page_scan, dim3((unsigned)scan_tiles(bin.key_space)), dim3(kScanThreads), 0, s, bin.key_space,
+    return launch_dependent(k_page_scan, dim3((unsigned)scan_tiles(bin.key_space)), dim3(kScanThreads), 0, s, bin.key_space,
                          (const uint8_t*)bin.grid_flag, bin.grid_rank, bin.grid_keys, (int)bin.ng_cap,
                          &cnt->n_grid_blocks, (uint8_t*)nullptr, scan.words + scan.grid, cnt);
 }
@@ -486,15 +491,15 @@ static cudaError_t launch_bin_sort(const BinDev& bin, const ScanScratch& scan, C
     const int64_t ncell = (int64_t)bin.nb_cap * 64;
     const int ilp = bin_ilp(bin.n), ctas = bin_ctas(bin.n, ilp);
     const unsigned hist = (unsigned)(ctas + (bin.grid_flag ? links_ctas(bin) : 0));
-    cudaError_t e = launch_kernel(ilp == kBinILP ? k_bin_hist_links<kBinILP> : k_bin_hist_links<kBinSmallILP>, dim3(hist), dim3(kBinThreads), 0, s, bin, (const Counters*)cnt);
+    cudaError_t e = launch_dependent(ilp == kBinILP ? k_bin_hist_links<kBinILP> : k_bin_hist_links<kBinSmallILP>, dim3(hist), dim3(kBinThreads), 0, s, bin, (const Counters*)cnt);
     if (e == cudaSuccess)
-        e = launch_kernel(k_cell_scan, dim3((unsigned)scan_tiles(ncell)), dim3(kScanThreads), 0, s, ncell, bin.cell_count,
+        e = launch_dependent(k_cell_scan, dim3((unsigned)scan_tiles(ncell)), dim3(kScanThreads), 0, s, ncell, bin.cell_count,
                           bin.cell_start, scan.words + scan.cells, clear_pages ? bin.page_flag : nullptr, bin.grid_flag,
                           bin.key_space, cnt);
     if (e == cudaSuccess)
-        e = launch_kernel(ilp == kBinILP ? k_bin_scatter<kBinILP> : k_bin_scatter<kBinSmallILP>, dim3((unsigned)ctas), dim3(kBinThreads), 0, s, bin);
+        e = launch_dependent(ilp == kBinILP ? k_bin_scatter<kBinILP> : k_bin_scatter<kBinSmallILP>, dim3((unsigned)ctas), dim3(kBinThreads), 0, s, bin);
     if (e == cudaSuccess)
-        e = launch_kernel(k_bin_canon, dim3((unsigned)canon_ctas(bin.nb_cap, num_sms)), dim3(32 * kCanonWarps), 0, s, bin,
+        e = launch_dependent(k_bin_canon, dim3((unsigned)canon_ctas(bin.nb_cap, num_sms)), dim3(32 * kCanonWarps), 0, s, bin,
                           scan, cnt);
     return e;
 }

@@ -622,6 +622,7 @@ template <typename R, bool kAnyModel, bool kFallback>
 __global__ void __launch_bounds__(kG2PUnit, sizeof(R) == 4 ? kG2PMinBlocks : 1)
     k_g2p(const SceneDev<R>* __restrict__ sc, const SceneDev<double>* __restrict__ sc64, PState<R> in,
           PState<R> out, PAux<R> aux, BinDev bin, const R* __restrict__ nodes, Counters* cnt) {
+    depend_on_previous();
     g2p_body<R, kAnyModel, kFallback>(own_blocks(), sc, sc64, in, out, aux, bin, nodes, cnt);
 }
 
@@ -641,6 +642,7 @@ __device__ __forceinline__ void advance_time_body(Counters* cnt, SceneDev<R>* sc
 
 template <typename R>
 __global__ void k_advance_time(Counters* cnt, SceneDev<R>* sc, SceneDev<double>* sc64) {
+    depend_on_previous();
     advance_time_body<R>(cnt, sc, sc64);
 }
 
@@ -714,19 +716,14 @@ cudaError_t launch_g2p(const SceneDev<R>* sc, const SceneDev<double>* sc64, cons
     const size_t smem = sizeof(G2PShared<R>);
     // FP64 state needs no FP64 fallback; FP32 launches the fallback form only where the scene has it
     const bool fb = sizeof(R) == 4 && fallback64 != nullptr;
-    if (cfg.other_models) {
-        if (fb)
-            k_g2p<R, true, (sizeof(R) == 4)><<<ctas, kG2PUnit, smem, stream>>>(sc, fallback64, in, out, aux, bin, nodes, cnt);
-        else
-            k_g2p<R, true, false><<<ctas, kG2PUnit, smem, stream>>>(sc, fallback64, in, out, aux, bin, nodes, cnt);
-    } else {
-        if (fb)
-            k_g2p<R, false, (sizeof(R) == 4)><<<ctas, kG2PUnit, smem, stream>>>(sc, fallback64, in, out, aux, bin, nodes, cnt);
-        else
-            k_g2p<R, false, false><<<ctas, kG2PUnit, smem, stream>>>(sc, fallback64, in, out, aux, bin, nodes, cnt);
-    }
-    k_advance_time<R><<<1, 1, 0, stream>>>(cnt, const_cast<SceneDev<R>*>(sc), const_cast<SceneDev<double>*>(sc64));
-    return cudaGetLastError();
+    auto* kernel = cfg.other_models ? (fb ? k_g2p<R, true, (sizeof(R) == 4)> : k_g2p<R, true, false>)
+                                    : (fb ? k_g2p<R, false, (sizeof(R) == 4)> : k_g2p<R, false, false>);
+    cudaError_t e = launch_dependent(kernel, dim3((unsigned)ctas), dim3(kG2PUnit), smem, stream, sc, fallback64, in, out, aux,
+                                     bin, nodes, cnt);
+    if (e == cudaSuccess)
+        e = launch_dependent(k_advance_time<R>, dim3(1), dim3(1), 0, stream, cnt, const_cast<SceneDev<R>*>(sc),
+                             const_cast<SceneDev<double>*>(sc64));
+    return e;
 }
 
 template cudaError_t launch_g2p<float>(const SceneDev<float>*, const SceneDev<double>*, const SceneDev<double>*,

@@ -152,6 +152,7 @@ template <typename R>
 __global__ void __launch_bounds__(kGridThreads)
     k_grid(const SceneDev<R>* __restrict__ sc, BinDev bin, const R* __restrict__ tile, R* __restrict__ nodes,
            double* __restrict__ diag, PcgDev pcg, Counters* cnt) {
+    depend_on_previous();
     grid_body<R>(own_blocks(), sc, bin, tile, nodes, diag, pcg, cnt);
 }
 
@@ -188,11 +189,10 @@ template cudaError_t launch_batch_grid<double>(const SceneArgs<double>*, const B
 template <typename R>
 cudaError_t launch_grid(const SceneDev<R>* sc, BinDev bin, GridDev grid, Counters* cnt, LaunchCfg cfg,
                         cudaStream_t stream) {
-    cudaMemsetAsync(grid.diag, 0, 4 * sizeof(double), stream);
     const int ctas = max(1, min(bin.ng_cap / 4 + 1, cfg.num_sms * 8));
-    k_grid<R><<<ctas, kGridThreads, 0, stream>>>(sc, bin, reinterpret_cast<const R*>(grid.tile),
-                                                 reinterpret_cast<R*>(grid.nodes), grid.diag, grid.pcg, cnt);
-    return cudaGetLastError();
+    return launch_dependent(k_grid<R>, dim3((unsigned)ctas), dim3(kGridThreads), 0, stream, sc, bin,
+                            reinterpret_cast<const R*>(grid.tile), reinterpret_cast<R*>(grid.nodes), grid.diag, grid.pcg,
+                            cnt);
 }
 
 template cudaError_t launch_grid<float>(const SceneDev<float>*, BinDev, GridDev, Counters*, LaunchCfg, cudaStream_t);

@@ -544,7 +544,10 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
 
 __global__ void __launch_bounds__(kP2GThreads, kCtasPerSm)
     k_p2g(const SceneDev<R>* __restrict__ sc, PState<R> st, PAux<R> aux, BinDev bin, R* __restrict__ tile,
-            Counters* __restrict__ cnt) {
+            Counters* __restrict__ cnt, double* __restrict__ diag) {
+    depend_on_previous();
+    // the sums that the grid stage adds to
+    if (blockIdx.x == 0 && threadIdx.x < 4) diag[threadIdx.x] = 0.0;
     p2g_body(own_blocks(), sc, st, aux, bin, tile, cnt);
 }
 
@@ -581,9 +584,8 @@ cudaError_t launch_batch_p2g<float>(const SceneArgs<float>* A, const BatchPlan& 
 template <>
 cudaError_t launch_p2g<float>(const SceneDev<float>* sc, const PState<float>& st, const PAux<float>& aux, BinDev bin,
                                GridDev grid, Counters* cnt, LaunchCfg cfg, cudaStream_t stream) {
-    k_p2g<<<p2g_ctas<float>(bin.nb_cap, cfg.num_sms), kP2GThreads, kSmem, stream>>>(
-        sc, st, aux, bin, reinterpret_cast<float*>(grid.tile), cnt);
-    return cudaGetLastError();
+    return launch_dependent(k_p2g, dim3((unsigned)p2g_ctas<float>(bin.nb_cap, cfg.num_sms)), dim3(kP2GThreads), kSmem, stream, sc, st,
+                            aux, bin, reinterpret_cast<float*>(grid.tile), cnt, grid.diag);
 }
 
 }  // namespace gmpm
