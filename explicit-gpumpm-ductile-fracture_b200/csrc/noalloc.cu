@@ -66,6 +66,41 @@ __global__ void k_noalloc_keys(int64_t n, const float* __restrict__ pos, double 
     page_flag[key >> 6] = 1;
 }
 
+// The same for many positions.  They come in any order, so their flag stores
+// would meet on the few active pages' bytes (94 us at 1M positions): a CTA
+// collects its pages in shared memory and adds them once, four flags a word.
+constexpr int kManyThreads = 1024;
+constexpr int64_t kMany = 1 << 16;  // below, clearing and scanning the CTA's flags costs more than it saves
+__global__ void __launch_bounds__(kManyThreads)
+    k_noalloc_keys_many(int64_t n, const float* __restrict__ pos, double inv_dx, int rx, int ry, int rz,
+                        uint32_t* __restrict__ keys, uint8_t* __restrict__ page_flag, Counters* cnt) {
+    __shared__ uint32_t seen[kNoAllocKeySpace / 4];
+    for (int w = threadIdx.x; w < (int)(kNoAllocKeySpace / 4); w += kManyThreads) seen[w] = 0u;
+    __syncthreads();
+    const int res[3] = {rx, ry, rz};
+    constexpr int kILP = 4;
+    const int64_t step = (int64_t)gridDim.x * kManyThreads;
+    bool bad = false;
+    for (int64_t i0 = (int64_t)blockIdx.x * kManyThreads + threadIdx.x; i0 < n; i0 += kILP * step) {
+        float x[kILP][3];
+#pragma unroll
+        for (int u = 0; u < kILP; ++u)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) x[u][a] = i0 + u * step < n ? pos[3 * (i0 + u * step) + a] : 0.f;
+#pragma unroll
+        for (int u = 0; u < kILP; ++u) {
+            if (i0 + u * step >= n) continue;
+            const uint32_t key = cell_key(x[u], inv_dx, res, bad);
+            keys[i0 + u * step] = key;
+            reinterpret_cast<uint8_t*>(seen)[key >> 6] = 1;
+        }
+    }
+    if (bad) raise_flag(cnt, GMPM_FLAG_OUT_OF_DOMAIN);
+    __syncthreads();
+    for (int w = threadIdx.x; w < (int)(kNoAllocKeySpace / 4); w += kManyThreads)
+        if (seen[w]) atomicOr(reinterpret_cast<uint32_t*>(page_flag) + w, seen[w]);
+}
+
 namespace {
 
 // Device address of g_noalloc_scratch per device, resolved on first use.
@@ -134,7 +169,10 @@ extern "C" gmpm_status gmpm_bin_positions_noalloc(const float* positions, int64_
     if (e == cudaSuccess) e = cudaMemsetAsync(scan.words, 0, scan.count * sizeof(uint32_t), s);
     const int T = 256;
     const unsigned gn = (unsigned)((n + T - 1) / T);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && n >= kMany)
+        e = launch_kernel(k_noalloc_keys_many, dim3((unsigned)sms), dim3(kManyThreads), 0, s, n, positions, 1.0 / dx, res_x,
+                          res_y, res_z, bin.keys, bin.page_flag, cnt);
+    else if (e == cudaSuccess)
         e = launch_kernel(k_noalloc_keys, dim3(gn), dim3(T), 0, s, n, positions, 1.0 / dx, res_x, res_y, res_z,
                           bin.keys, bin.page_flag, cnt);
     if (e == cudaSuccess) e = launch_bin_no_grid(bin, scan, cnt, sms, s);
