@@ -112,10 +112,17 @@ __device__ __forceinline__ void page_scan_body(uint32_t key_space, const uint8_t
             over = true;
         ++run;
         if (grid_flag) {
-            int bx, by, bz;
-            page_coords(k, bx, by, bz);
+            // the next coordinate along an axis is an increment of the key's interleaved bits of that axis
+            // (decoding the key and interleaving eight took most of the scan's time)
+            constexpr uint32_t kAxis[3] = {0x24924924u, 0x12492492u, 0x09249249u};
+            uint32_t c[3][2];
 #pragma unroll
-            for (int d = 0; d < 8; ++d) grid_flag[page_key(bx + (d >> 2), by + ((d >> 1) & 1), bz + (d & 1))] = 1;
+            for (int a = 0; a < 3; ++a) {
+                c[a][0] = k & kAxis[a];
+                c[a][1] = ((k | ~kAxis[a]) + 1) & kAxis[a];
+            }
+#pragma unroll
+            for (int d = 0; d < 8; ++d) grid_flag[c[0][d >> 2] | c[1][(d >> 1) & 1] | c[2][d & 1]] = 1;
         }
     }
     if (over) raise_flag(cnt, GMPM_FLAG_TABLE_OVERFLOW);
