@@ -302,7 +302,7 @@ struct Scene : SceneBase {
             if (rstage_free_[b]) cudaEventDestroy(rstage_free_[b]);
         }
         if (copy_stream_) cudaStreamDestroy(copy_stream_);
-        if (pcg_done_host) cudaFreeHost(pcg_done_host);
+        if (pcg_host) cudaFreeHost(pcg_host);
         if (bc_staging) cudaFreeHost(bc_staging);
         if (dt_staging) cudaFreeHost(dt_staging);
         for (cudaEvent_t e : dt_done)
@@ -329,7 +329,8 @@ struct Scene : SceneBase {
                          desc.pcg_max_combine, desc.materials[0].mobility, desc.pcg_tolerance, other};
     }
     bool implicit_pf() const { return desc.phase_field == GMPM_PHASE_FIELD_IMPLICIT; }
-    int* pcg_done_host = nullptr;  // pinned: the solve's done flag, read between iterations
+    PcgScalars* pcg_host = nullptr;  // pinned: the solve's scalars, read between iterations
+    int pcg_first_check = 4;         // iterations before the first read
 
     gmpm_status create(gmpm_context* c, const gmpm_scene_desc* d, const gmpm_particle_init* init) {
         ctx = c;
@@ -495,7 +496,7 @@ struct Scene : SceneBase {
             GMPM_TRY(alloc(&P.scal, 1));
             GMPM_TRY(cudaMemset(P.scal, 0, sizeof(PcgScalars)));
             P.n = n;
-            GMPM_TRY(cudaMallocHost(reinterpret_cast<void**>(&pcg_done_host), sizeof(int)));
+            GMPM_TRY(cudaMallocHost(reinterpret_cast<void**>(&pcg_host), sizeof(PcgScalars)));
         }
         GMPM_TRY(prepare_p2g<R>());
         GMPM_TRY(prepare_g2p<R>());
@@ -551,7 +552,7 @@ struct Scene : SceneBase {
     // Kernels of one substep from state buffer c; ev (optional) receives
     // events after bin, p2g, grid (incl. an implicit phase-field solve), g2p.
     // Host bookkeeping is left alone.  host_checks: the implicit solve reads
-    // its done flag every 4 iterations and stops launching (not when capturing).
+    // its done flag between iterations and stops launching (not when capturing).
     gmpm_status launch_one(cudaStream_t s, int c, cudaEvent_t* ev, bool host_checks = true,
                            int64_t* kernels = nullptr) {
         const LaunchCfg lc = cfg();
@@ -569,11 +570,16 @@ struct Scene : SceneBase {
             for (int it = 0; it < desc.pcg_max_iterations; ++it) {
                 GMPM_TRY(launch_pcg_iteration<R>(d_sc, st[c], aux, bin, grid, d_cnt, lc, s));
                 nk += kPcgIterationKernels;
-                if (host_checks && (it & 3) == 3) {
-                    GMPM_TRY(cudaMemcpyAsync(pcg_done_host, &grid.pcg.scal->done, sizeof(int),
-                                             cudaMemcpyDeviceToHost, s));
+                // The done flag is first read after as many iterations as the last solve took (kernels of a
+                // converged solve return at once, but 21 of them cost as much as an iteration of a small
+                // scene), then every 4.
+                if (host_checks && it + 1 >= pcg_first_check && ((it + 1 - pcg_first_check) & 3) == 0) {
+                    GMPM_TRY(cudaMemcpyAsync(pcg_host, grid.pcg.scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s));
                     GMPM_TRY(cudaStreamSynchronize(s));
-                    if (*pcg_done_host) break;
+                    if (pcg_host->done) {
+                        pcg_first_check = std::max(1, pcg_host->iterations);
+                        break;
+                    }
                 }
             }
             GMPM_TRY(launch_pcg_finish<R>(d_sc, bin, grid, d_cnt, lc, s));

@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace gmpm {
 
@@ -105,6 +106,7 @@ __device__ double combine_partials(const double* part, int n, bool use_max, doub
 __global__ void __launch_bounds__(kPcgBlock)
     k_pcg_dot(const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ part, BinDev bin,
               const Counters* __restrict__ cnt) {
+    depend_on_previous();
     __shared__ double sh[32];
     const int N = pcg_entries(cnt, bin);
     const int nparts = (N + kPcgBlock - 1) / kPcgBlock;
@@ -118,6 +120,7 @@ __global__ void __launch_bounds__(kPcgBlock)
 
 __global__ void __launch_bounds__(kPcgScalarThreads)
     k_pcg_start(PcgDev P, BinDev bin, Counters* cnt, int max_combine) {
+    depend_on_previous();
     __shared__ double sh[32];
     const int N = pcg_entries(cnt, bin);
     const double rho = combine_partials(P.part, (N + kPcgBlock - 1) / kPcgBlock, max_combine != 0, sh);
@@ -136,6 +139,7 @@ template <typename R>
 __global__ void __launch_bounds__(kPcgColThreads)
     k_pcg_col(const SceneDev<R>* __restrict__ sc, PState<R> st, PAux<R> aux, BinDev bin, PcgDev P,
               const Counters* __restrict__ cnt) {
+    depend_on_previous();
     if (P.scal->done) return;
     __shared__ double win[kWindowNodes];
     const int nb = min(cnt->n_blocks, bin.nb_cap);
@@ -256,6 +260,7 @@ template <typename R>
 __global__ void __launch_bounds__(kPcgKxThreads, 4)
     k_pcg_kx(const SceneDev<R>* __restrict__ sc, PState<R> st, BinDev bin, PcgDev P, double* __restrict__ tile,
              const Counters* __restrict__ cnt) {
+    depend_on_previous();
     if (P.scal->done) return;
     __shared__ double recs[kPcgKxChunk * kKxRec];  // staged particles; the column sums at a page's end
     __shared__ int cstart[65];
@@ -350,6 +355,7 @@ __global__ void __launch_bounds__(kPcgKxThreads, 4)
 __global__ void __launch_bounds__(kPcgBlock)
     k_pcg_q(BinDev bin, PcgDev P, const double* __restrict__ tile, const Counters* __restrict__ cnt,
             double mobility) {
+    depend_on_previous();
     if (P.scal->done) return;
     __shared__ double sh[32];
     const int N = pcg_entries(cnt, bin);
@@ -381,6 +387,7 @@ __global__ void __launch_bounds__(kPcgBlock)
 
 __global__ void __launch_bounds__(kPcgScalarThreads)
     k_pcg_alpha(PcgDev P, BinDev bin, const Counters* __restrict__ cnt, int max_combine) {
+    depend_on_previous();
     if (P.scal->done) return;
     __shared__ double sh[32];
     const int N = pcg_entries(cnt, bin);
@@ -392,6 +399,7 @@ __global__ void __launch_bounds__(kPcgScalarThreads)
 // partial max r^2 and partial sums of r . mr
 __global__ void __launch_bounds__(kPcgBlock)
     k_pcg_update(BinDev bin, PcgDev P, const Counters* __restrict__ cnt) {
+    depend_on_previous();
     if (P.scal->done) return;
     __shared__ double sh[32];
     const int N = pcg_entries(cnt, bin);
@@ -429,6 +437,7 @@ __global__ void __launch_bounds__(kPcgBlock)
 // residual norm, convergence, rho and the direction update rate
 __global__ void __launch_bounds__(kPcgScalarThreads)
     k_pcg_rho(PcgDev P, BinDev bin, const Counters* __restrict__ cnt, int max_combine, double tol) {
+    depend_on_previous();
     if (P.scal->done) return;
     __shared__ double sh[32];
     const int N = pcg_entries(cnt, bin);
@@ -455,6 +464,7 @@ __global__ void __launch_bounds__(kPcgScalarThreads)
 
 // s = s rate + mr on tagged nodes (cal_grid_r_vad_kernal)
 __global__ void __launch_bounds__(kPcgBlock) k_pcg_sdir(BinDev bin, PcgDev P, const Counters* __restrict__ cnt) {
+    depend_on_previous();
     if (P.scal->done) return;
     const int N = pcg_entries(cnt, bin);
     const double rate = P.scal->rate;
@@ -466,6 +476,7 @@ __global__ void __launch_bounds__(kPcgBlock) k_pcg_sdir(BinDev bin, PcgDev P, co
 // x = 1e20 everywhere after a breakdown (rho_old == 0)
 template <typename R>
 __global__ void k_pcg_finish(BinDev bin, PcgDev P, R* __restrict__ nodes, Counters* cnt) {
+    depend_on_previous();
     const int N = pcg_entries(cnt, bin);
     const bool blow = P.scal->blowup != 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
@@ -492,9 +503,10 @@ template <typename R>
 cudaError_t launch_pcg_init(const SceneDev<R>* sc, BinDev bin, GridDev grid, Counters* cnt, LaunchCfg cfg,
                             cudaStream_t stream) {
     const PcgDev& P = grid.pcg;
-    k_pcg_dot<<<pcg_grid_blocks(bin, cfg), kPcgBlock, 0, stream>>>(P.r, P.mr, P.part, bin, cnt);
-    k_pcg_start<<<1, kPcgScalarThreads, 0, stream>>>(P, bin, cnt, cfg.pcg_max_combine);
-    return cudaGetLastError();
+    const dim3 gb((unsigned)pcg_grid_blocks(bin, cfg)), block(kPcgBlock), one(1), scalar(kPcgScalarThreads);
+    cudaError_t e = launch_dependent(k_pcg_dot, gb, block, 0, stream, P.r, P.mr, P.part, bin, cnt);
+    if (e == cudaSuccess) e = launch_dependent(k_pcg_start, one, scalar, 0, stream, P, bin, cnt, cfg.pcg_max_combine);
+    return e;
 }
 
 template <typename R>
@@ -502,24 +514,24 @@ cudaError_t launch_pcg_iteration(const SceneDev<R>* sc, const PState<R>& st, con
                                  GridDev grid, Counters* cnt, LaunchCfg cfg, cudaStream_t stream) {
     const PcgDev& P = grid.pcg;
     double* tile = reinterpret_cast<double*>(grid.tile);
-    const int pages = max(1, min(bin.nb_cap, cfg.num_sms * 4));
-    const int gb = pcg_grid_blocks(bin, cfg);
-    k_pcg_col<R><<<pages, kPcgColThreads, 0, stream>>>(sc, st, aux, bin, P, cnt);
-    k_pcg_kx<R><<<max(1, min(bin.nb_cap, cfg.num_sms * 8)), kPcgKxThreads, 0, stream>>>(sc, st, bin, P, tile, cnt);
-    k_pcg_q<<<gb, kPcgBlock, 0, stream>>>(bin, P, tile, cnt, cfg.pcg_mobility);
-    k_pcg_alpha<<<1, kPcgScalarThreads, 0, stream>>>(P, bin, cnt, cfg.pcg_max_combine);
-    k_pcg_update<<<gb, kPcgBlock, 0, stream>>>(bin, P, cnt);
-    k_pcg_rho<<<1, kPcgScalarThreads, 0, stream>>>(P, bin, cnt, cfg.pcg_max_combine, cfg.pcg_tolerance);
-    k_pcg_sdir<<<gb, kPcgBlock, 0, stream>>>(bin, P, cnt);
-    return cudaGetLastError();
+    const dim3 col((unsigned)max(1, min(bin.nb_cap, cfg.num_sms * 4))), kx((unsigned)max(1, min(bin.nb_cap, cfg.num_sms * 8)));
+    const dim3 gb((unsigned)pcg_grid_blocks(bin, cfg)), block(kPcgBlock), one(1), scalar(kPcgScalarThreads);
+    cudaError_t e = launch_dependent(k_pcg_col<R>, col, dim3(kPcgColThreads), 0, stream, sc, st, aux, bin, P, cnt);
+    if (e == cudaSuccess) e = launch_dependent(k_pcg_kx<R>, kx, dim3(kPcgKxThreads), 0, stream, sc, st, bin, P, tile, cnt);
+    if (e == cudaSuccess) e = launch_dependent(k_pcg_q, gb, block, 0, stream, bin, P, tile, cnt, cfg.pcg_mobility);
+    if (e == cudaSuccess) e = launch_dependent(k_pcg_alpha, one, scalar, 0, stream, P, bin, cnt, cfg.pcg_max_combine);
+    if (e == cudaSuccess) e = launch_dependent(k_pcg_update, gb, block, 0, stream, bin, P, cnt);
+    if (e == cudaSuccess)
+        e = launch_dependent(k_pcg_rho, one, scalar, 0, stream, P, bin, cnt, cfg.pcg_max_combine, cfg.pcg_tolerance);
+    if (e == cudaSuccess) e = launch_dependent(k_pcg_sdir, gb, block, 0, stream, bin, P, cnt);
+    return e;
 }
 
 template <typename R>
 cudaError_t launch_pcg_finish(const SceneDev<R>* sc, BinDev bin, GridDev grid, Counters* cnt, LaunchCfg cfg,
                               cudaStream_t stream) {
-    k_pcg_finish<R><<<pcg_grid_blocks(bin, cfg), kPcgBlock, 0, stream>>>(bin, grid.pcg,
-                                                                         reinterpret_cast<R*>(grid.nodes), cnt);
-    return cudaGetLastError();
+    return launch_dependent(k_pcg_finish<R>, dim3((unsigned)pcg_grid_blocks(bin, cfg)), dim3(kPcgBlock), 0, stream, bin,
+                            grid.pcg, reinterpret_cast<R*>(grid.nodes), cnt);
 }
 
 #define GMPM_PCG_INST(R)                                                                                            \
