@@ -1,6 +1,7 @@
 // Scene initialisation (first constitutive evaluation), FP64 particle
 // diagnostics and field readback.
 #include <cstdint>
+#include <type_traits>
 
 #include "constitutive.cuh"
 #include "kernels.h"
@@ -111,6 +112,9 @@ template cudaError_t launch_particle_diag<double>(const PState<double>&, const P
 
 // ---------------------------------------------------------------------------
 
+constexpr int kPackThreads = 256;
+__host__ __device__ constexpr int pack_ilp(int nc) { return nc <= 1 ? 8 : nc <= 3 ? 4 : 2; }
+
 struct FieldPlanes {
     const void* plane[9];
     int step[9];  // elements between particles: 1 for a plane, 4 for a component of a four-wide word
@@ -152,26 +156,34 @@ __host__ FieldPlanes field_planes(const PState<R>& st, const PAux<R>& aux, int f
     return f;
 }
 
-template <typename R>
-__global__ void k_pack_field(FieldPlanes f, const uint32_t* __restrict__ ids, int dtype, int order, int64_t n,
-                             void* out) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const int64_t dst = (order == GMPM_ORDER_ORIGINAL) ? (int64_t)(ids[p] & 0x0fffffffu) : p;
-    if (dst >= n) return;
-    for (int q = 0; q < f.comps; ++q) {
-        double v;
-        if (f.is_id)
-            v = (double)(reinterpret_cast<const uint32_t*>(f.plane[q])[p] & 0x0fffffffu);
-        else
-            v = (double)reinterpret_cast<const R*>(f.plane[q])[p * f.step[q]];
-        const int64_t e = dst * f.comps + q;
-        if (dtype == GMPM_DTYPE_F64)
-            reinterpret_cast<double*>(out)[e] = v;
-        else if (dtype == GMPM_DTYPE_F32)
-            reinterpret_cast<float*>(out)[e] = (float)v;
-        else
-            reinterpret_cast<int32_t*>(out)[e] = (int32_t)v;
+// A field of NC components in the caller's type and order.  A thread takes
+// kILP particles a CTA width apart and has all their values (and places) under
+// way before it writes the first: one value at a time, each a round trip of
+// its own, a position and a damage read of 8.4M particles took 1.4 ms.
+template <typename R, int NC, typename T>
+__global__ void __launch_bounds__(kPackThreads) k_pack_field(FieldPlanes f, const uint32_t* __restrict__ ids, int order,
+                                                             int64_t n, T* __restrict__ out) {
+    constexpr int kILP = pack_ilp(NC);
+    const int64_t p0 = (int64_t)blockIdx.x * kPackThreads * kILP + threadIdx.x;
+    int64_t dst[kILP];
+    double v[kILP][NC];  // R to T through double, as the values' one conversion
+#pragma unroll
+    for (int u = 0; u < kILP; ++u) {
+        const int64_t p = p0 + (int64_t)u * kPackThreads;
+        dst[u] = p >= n ? n : order == GMPM_ORDER_ORIGINAL ? (int64_t)(ids[p] & 0x0fffffffu) : p;
+        if (p >= n) continue;
+        if (NC == 1 && f.is_id) {
+            v[u][0] = (double)(reinterpret_cast<const uint32_t*>(f.plane[0])[p] & 0x0fffffffu);
+        } else {
+#pragma unroll
+            for (int q = 0; q < NC; ++q) v[u][q] = (double)reinterpret_cast<const R*>(f.plane[q])[p * f.step[q]];
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kILP; ++u) {
+        if (dst[u] >= n) continue;
+#pragma unroll
+        for (int q = 0; q < NC; ++q) out[dst[u] * NC + q] = (T)v[u][q];
     }
 }
 
@@ -189,9 +201,27 @@ int field_components(int field) {
 template <typename R>
 cudaError_t launch_pack_field(const PState<R>& st, const PAux<R>& aux, int field, int dtype, int order, int64_t n,
                               void* out, cudaStream_t stream) {
-    FieldPlanes f = field_planes(st, aux, field);
-    const int T = 256;
-    k_pack_field<R><<<(unsigned)((n + T - 1) / T), T, 0, stream>>>(f, st.id, dtype, order, n, out);
+    const FieldPlanes f = field_planes(st, aux, field);
+    auto launch = [&](auto nc, auto* dst) {
+        constexpr int NC = decltype(nc)::value;
+        const int64_t per = (int64_t)kPackThreads * pack_ilp(NC);
+        k_pack_field<R, NC><<<(unsigned)((n + per - 1) / per), kPackThreads, 0, stream>>>(f, st.id, order, n, dst);
+    };
+    auto typed = [&](auto nc) {
+        if (dtype == GMPM_DTYPE_F64)
+            launch(nc, reinterpret_cast<double*>(out));
+        else if (dtype == GMPM_DTYPE_F32)
+            launch(nc, reinterpret_cast<float*>(out));
+        else
+            launch(nc, reinterpret_cast<int32_t*>(out));
+    };
+    switch (f.comps) {
+        case 1: typed(std::integral_constant<int, 1>{}); break;
+        case 3: typed(std::integral_constant<int, 3>{}); break;
+        case 6: typed(std::integral_constant<int, 6>{}); break;
+        case 9: typed(std::integral_constant<int, 9>{}); break;
+        default: break;
+    }
     return cudaGetLastError();
 }
 template cudaError_t launch_pack_field<float>(const PState<float>&, const PAux<float>&, int, int, int, int64_t,
