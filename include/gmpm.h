@@ -146,7 +146,7 @@ typedef struct gmpm_scene_desc {
     gmpm_sphere_bc spheres[GMPM_MAX_SPHERE_BCS];
     int32_t precision;         /* gmpm_precision */
     int32_t phase_field;       /* gmpm_phase_field */
-    int32_t deterministic;     /* 1 = fixed-order P2G (bitwise reproducible), 0 = atomic fast mode */
+    int32_t deterministic;     /* 1 = bitwise reproducible; 0 = not asked for (both run the fixed-order P2G) */
     int32_t block_capacity;    /* max active pages; 0 = derive from the particle count */
     double svd_fallback_ratio; /* sigma_min/sigma_max threshold for the FP64 fallback (1e-3) */
     int32_t adaptive_dt;       /* 1: each substep's dt = min(dt, cfl_number dx / max |v_p|), computed on the
