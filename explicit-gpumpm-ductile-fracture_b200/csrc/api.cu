@@ -520,6 +520,7 @@ struct Scene : SceneBase {
         Counters h{};
         cudaError_t e = cudaMemcpy(&h, d_cnt, sizeof(h), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return e;
+        if (h.flags & GMPM_FLAG_COPY_TIMEOUT) return cudaErrorTimeout;  // a scan gave up: no counts
         *nb = h.n_blocks;
         *ng = h.n_grid_blocks;
         return cudaGetLastError();

@@ -75,16 +75,28 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_keys(int64_t n, const R* __
     bin_keys_body<R>(own_blocks(), n, x0, x1, x2, sc, keys, page_flag, cnt);
 }
 
+// A wait of a scan gave up: ranks, counts or starts are not to be used.  The
+// rest of the binning then does nothing but restore its working words, and
+// without pages the substep's other kernels do nothing.
+__device__ __forceinline__ void scan_gave_up(uint32_t* failed, Counters* cnt) {
+    *failed = 1u;
+    raise_flag(cnt, GMPM_FLAG_COPY_TIMEOUT);
+}
+// The page scan found pages and no wait gave up (n >= 1, so there are pages).
+__device__ __forceinline__ bool scans_done(const ScanScratch& scan, const Counters* cnt) {
+    return scan.words[scan.count - 1] == 0u && cnt->n_blocks > 0;
+}
+
 // Ranks of the flagged keys in ascending order, with their list and count:
 // page ids (the first scan) or grid page ids (the second).  The first also
 // marks every active page and its 7 "+" neighbours as grid pages
 // (supplementAdjacentPages, Transformer_kernal.cu:70-96).  words: the scan's
 // status words and, after them, its ticket.  Ranks of keys without a flag are
-// left as they are; no reader looks at them.
+// left as they are; no reader looks at them.  failed: set where a wait gave up.
 __device__ __forceinline__ void page_scan_body(uint32_t key_space, const uint8_t* __restrict__ flag,
                                                int32_t* __restrict__ rank, uint32_t* __restrict__ list, int cap,
                                                int32_t* __restrict__ total, uint8_t* __restrict__ grid_flag,
-                                               uint32_t* __restrict__ words, Counters* cnt) {
+                                               uint32_t* __restrict__ words, uint32_t* failed, Counters* cnt) {
     const int ntiles = (int)((key_space + kScanTile - 1) / kScanTile);
     const int tile = scan_take_tile(words + ntiles);
     if (tile >= ntiles) return;
@@ -126,18 +138,18 @@ __device__ __forceinline__ void page_scan_body(uint32_t key_space, const uint8_t
         }
     }
     if (over) raise_flag(cnt, GMPM_FLAG_TABLE_OVERFLOW);
-    if (tile == ntiles - 1 && threadIdx.x == 0) {
-        *total = bad ? 0 : before + tot;  // without a count nothing downstream runs
-        if (bad) raise_flag(cnt, GMPM_FLAG_COPY_TIMEOUT);
+    if (threadIdx.x == 0) {
+        if (tile == ntiles - 1) *total = before + tot;
+        if (bad) scan_gave_up(failed, cnt);
     }
 }
 
 __global__ void __launch_bounds__(kScanThreads)
     k_page_scan(uint32_t key_space, const uint8_t* __restrict__ flag, int32_t* __restrict__ rank,
                 uint32_t* __restrict__ list, int cap, int32_t* __restrict__ total, uint8_t* __restrict__ grid_flag,
-                uint32_t* __restrict__ words, Counters* cnt) {
+                uint32_t* __restrict__ words, uint32_t* failed, Counters* cnt) {
     depend_on_previous();
-    page_scan_body(key_space, flag, rank, list, cap, total, grid_flag, words, cnt);
+    page_scan_body(key_space, flag, rank, list, cap, total, grid_flag, words, failed, cnt);
 }
 
 // Zero `bytes` (a multiple of 16, from a 16-byte boundary) in 4 KiB pieces: pieces vb.b, vb.b + vb.g, ...
@@ -152,12 +164,16 @@ __device__ __forceinline__ void zero_bytes_body(VB vb, void* p, int64_t bytes) {
 // pointers.  clear: flags whose last use in the binning was the page links,
 // cleared here for the next one (or null).
 __device__ __forceinline__ void cell_scan_body(VB vb, int64_t ncell, int32_t* __restrict__ count,
-                                               int32_t* __restrict__ start, uint32_t* __restrict__ words,
+                                               int32_t* __restrict__ start, const ScanScratch& scan,
                                                uint8_t* clear0, uint8_t* clear1, uint32_t key_space, Counters* cnt) {
     if (clear0) zero_bytes_body(vb, clear0, key_space);
     if (clear1) zero_bytes_body(vb, clear1, key_space);
-    const int64_t m = min(ncell, (int64_t)max(cnt->n_blocks, 0) * 64);
-    const int tile = scan_take_tile(words + (ncell + kScanTile - 1) / kScanTile);
+    uint32_t* words = scan.words + scan.cells;
+    // read once per CTA: a peer that gives up may set the failure word meanwhile
+    __shared__ int64_t live;
+    if (threadIdx.x == 0) live = scans_done(scan, cnt) ? min(ncell, (int64_t)cnt->n_blocks * 64) : 0;
+    const int tile = scan_take_tile(words + (ncell + kScanTile - 1) / kScanTile);  // with a barrier
+    const int64_t m = live;
     const int64_t base = (int64_t)tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
     if ((int64_t)tile * kScanTile >= max(m, (int64_t)1)) return;  // whole CTA; tile 0 writes the total of no cells
     int4 v[kScanItems / 4];
@@ -182,20 +198,17 @@ __device__ __forceinline__ void cell_scan_body(VB vb, int64_t ncell, int32_t* __
         }
         run = o.w + v[q].w;
     }
-    if (threadIdx.x == 0 && m <= (int64_t)(tile + 1) * kScanTile) {  // the tile of the last live cell
-        start[m] = before + tot;
-        if (bad) {
-            cnt->n_blocks = 0;
-            raise_flag(cnt, GMPM_FLAG_COPY_TIMEOUT);
-        }
+    if (threadIdx.x == 0) {
+        if (m <= (int64_t)(tile + 1) * kScanTile) start[m] = before + tot;  // the tile of the last live cell
+        if (bad) scan_gave_up(scan.words + scan.count - 1, cnt);
     }
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-    k_cell_scan(int64_t ncell, int32_t* __restrict__ count, int32_t* __restrict__ start, uint32_t* __restrict__ words,
+    k_cell_scan(int64_t ncell, int32_t* __restrict__ count, int32_t* __restrict__ start, ScanScratch scan,
                 uint8_t* clear0, uint8_t* clear1, uint32_t key_space, Counters* cnt) {
     depend_on_previous();
-    cell_scan_body(own_blocks(), ncell, count, start, words, clear0, clear1, key_space, cnt);
+    cell_scan_body(own_blocks(), ncell, count, start, scan, clear0, clear1, key_space, cnt);
 }
 
 // Page topology: adj (establishPageTopology, Transformer_kernal.cu:98-114) and
@@ -257,8 +270,9 @@ __host__ __device__ inline int bin_ctas(int64_t n, int ilp) {
 
 // The histogram's CTAs and, after them, the page links' (both need the ranks only).
 template <int kILP>
-__global__ void __launch_bounds__(kBinThreads) k_bin_hist_links(BinDev bin, const Counters* cnt) {
+__global__ void __launch_bounds__(kBinThreads) k_bin_hist_links(BinDev bin, ScanScratch scan, const Counters* cnt) {
     depend_on_previous();
+    if (!scans_done(scan, cnt)) return;
     const VB vb = own_blocks();
     const int hist = bin_ctas(bin.n, kILP);
     if (vb.b < hist)
@@ -304,8 +318,12 @@ __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_
 }
 
 template <int kILP>
-__global__ void __launch_bounds__(kBinThreads) k_bin_scatter(BinDev bin) {
+__global__ void __launch_bounds__(kBinThreads) k_bin_scatter(BinDev bin, ScanScratch scan, Counters* cnt) {
     depend_on_previous();
+    if (!scans_done(scan, cnt)) {  // without starts the counts are no fill pointers; no pages for the kernels after
+        if (blockIdx.x == 0 && threadIdx.x == 0) cnt->n_blocks = cnt->n_grid_blocks = 0;
+        return;
+    }
     bin_scatter_body<kILP, false>(own_blocks(), bin.n, bin.keys, bin.page_rank, nullptr, bin.cell_count, bin.perm,
                                   bin.keys_sorted, bin.nb_cap);
 }
@@ -401,7 +419,9 @@ __device__ __forceinline__ void canon_rank_warp(const BinDev& bin, const int32_t
         }
 }
 
-// Also clears, for the next binning, the fill pointers of the pages' cells and the scans' words.
+// Also clears, for the next binning, the fill pointers of the pages' cells
+// (without pages, after a scan that gave up, those of every cell: the
+// histogram may have run) and the scans' words.
 __device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, const ScanScratch& scan, Counters* cnt) {
     __shared__ int32_t buf[kCanonBuf];
     __shared__ int32_t cs[kCanonWarps][68];
@@ -414,6 +434,7 @@ __device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, const S
     int32_t* wbuf = buf + warp * kCanonWarpBuf;
     if (vb.b == 0)
         for (int q = threadIdx.x; q < scan.count; q += blockDim.x) scan.words[q] = 0u;
+    if (nb <= 0) zero_bytes_body(vb, bin.cell_count, (int64_t)bin.nb_cap * 64 * 4);
     for (int g = vb.b * kCanonWarps; g < nb; g += vb.g * kCanonWarps) {
         const int b = g + warp;
         int is_big = 0;
@@ -479,12 +500,12 @@ static int links_ctas(const BinDev& bin) { return (int)(((int64_t)std::max(bin.n
 static cudaError_t launch_page_scan(const BinDev& bin, const ScanScratch& scan, Counters* cnt, bool mark, cudaStream_t s) {
     return launch_dependent(k_page_scan, dim3((unsigned)scan_tiles(bin.key_space)), dim3(kScanThreads), 0, s, bin.key_space,
                          (const uint8_t*)bin.page_flag, bin.page_rank, bin.block_keys, (int)bin.nb_cap, &cnt->n_blocks,
-                         mark ? bin.grid_flag : nullptr, scan.words, cnt);
+                         mark ? bin.grid_flag : nullptr, scan.words, scan.words + scan.count - 1, cnt);
 }
 static cudaError_t launch_grid_scan(const BinDev& bin, const ScanScratch& scan, Counters* cnt, cudaStream_t s) {
     return launch_dependent(k_page_scan, dim3((unsigned)scan_tiles(bin.key_space)), dim3(kScanThreads), 0, s, bin.key_space,
                          (const uint8_t*)bin.grid_flag, bin.grid_rank, bin.grid_keys, (int)bin.ng_cap,
-                         &cnt->n_grid_blocks, (uint8_t*)nullptr, scan.words + scan.grid, cnt);
+                         &cnt->n_grid_blocks, (uint8_t*)nullptr, scan.words + scan.grid, scan.words + scan.count - 1, cnt);
 }
 
 cudaError_t launch_page_scans(BinDev bin, ScanScratch scan, Counters* cnt, cudaStream_t s) {
@@ -498,13 +519,13 @@ static cudaError_t launch_bin_sort(const BinDev& bin, const ScanScratch& scan, C
     const int64_t ncell = (int64_t)bin.nb_cap * 64;
     const int ilp = bin_ilp(bin.n), ctas = bin_ctas(bin.n, ilp);
     const unsigned hist = (unsigned)(ctas + (bin.grid_flag ? links_ctas(bin) : 0));
-    cudaError_t e = launch_dependent(ilp == kBinILP ? k_bin_hist_links<kBinILP> : k_bin_hist_links<kBinSmallILP>, dim3(hist), dim3(kBinThreads), 0, s, bin, (const Counters*)cnt);
+    cudaError_t e = launch_dependent(ilp == kBinILP ? k_bin_hist_links<kBinILP> : k_bin_hist_links<kBinSmallILP>, dim3(hist), dim3(kBinThreads), 0, s, bin, scan, (const Counters*)cnt);
     if (e == cudaSuccess)
         e = launch_dependent(k_cell_scan, dim3((unsigned)scan_tiles(ncell)), dim3(kScanThreads), 0, s, ncell, bin.cell_count,
-                          bin.cell_start, scan.words + scan.cells, clear_pages ? bin.page_flag : nullptr, bin.grid_flag,
+                          bin.cell_start, scan, clear_pages ? bin.page_flag : nullptr, bin.grid_flag,
                           bin.key_space, cnt);
     if (e == cudaSuccess)
-        e = launch_dependent(ilp == kBinILP ? k_bin_scatter<kBinILP> : k_bin_scatter<kBinSmallILP>, dim3((unsigned)ctas), dim3(kBinThreads), 0, s, bin);
+        e = launch_dependent(ilp == kBinILP ? k_bin_scatter<kBinILP> : k_bin_scatter<kBinSmallILP>, dim3((unsigned)ctas), dim3(kBinThreads), 0, s, bin, scan, cnt);
     if (e == cudaSuccess)
         e = launch_dependent(k_bin_canon, dim3((unsigned)canon_ctas(bin.nb_cap, num_sms)), dim3(32 * kCanonWarps), 0, s, bin,
                           scan, cnt);
@@ -689,7 +710,9 @@ template <typename R>
 __global__ void __launch_bounds__(kBinThreads) k_batch_hist(const SceneArgs<R>* __restrict__ A,
                                                             const int32_t* __restrict__ start, int ns) {
     VB vb;
-    const BinDev& bin = A[scene_of_block(start, ns, vb)].bin;
+    const SceneArgs<R>& a = A[scene_of_block(start, ns, vb)];
+    if (a.cnt->n_blocks <= 0) return;  // no page has a flag (a binning before gave up): ranks and starts are not its own
+    const BinDev& bin = a.bin;
     bin_hist_body<kBinILP>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap);
 }
 
@@ -697,7 +720,9 @@ template <typename R>
 __global__ void __launch_bounds__(kBinThreads) k_batch_scatter(const SceneArgs<R>* __restrict__ A,
                                                                const int32_t* __restrict__ start, int ns) {
     VB vb;
-    const BinDev& bin = A[scene_of_block(start, ns, vb)].bin;
+    const SceneArgs<R>& a = A[scene_of_block(start, ns, vb)];
+    if (a.cnt->n_blocks <= 0) return;
+    const BinDev& bin = a.bin;
     bin_scatter_body<kBinILP, true>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_start, bin.cell_count, bin.perm, bin.keys_sorted,
                      bin.nb_cap);
 }

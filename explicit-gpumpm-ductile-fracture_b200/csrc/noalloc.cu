@@ -43,9 +43,9 @@ constexpr size_t kOffBlockKeys = align256(kOffPageRank + kNoAllocKeySpace * size
 constexpr size_t kOffCellCount = align256(kOffBlockKeys + kNoAllocKeySpace * sizeof(uint32_t));
 constexpr size_t kOffCellStart = align256(kOffCellCount + kNoAllocCells * sizeof(int32_t));
 constexpr size_t kOffScanTiles = align256(kOffCellStart + (kNoAllocCells + 1) * sizeof(int32_t));
-// status words of the page scan, an unused grid scan and the cell scan, with their tickets
+// status words of the page scan, an unused grid scan and the cell scan, with their tickets; the failure word
 constexpr size_t kScanWords =
-    2 * ((kNoAllocKeySpace + kScanTile - 1) / kScanTile + 1) + (kNoAllocCells + kScanTile - 1) / kScanTile + 1;
+    2 * ((kNoAllocKeySpace + kScanTile - 1) / kScanTile + 1) + (kNoAllocCells + kScanTile - 1) / kScanTile + 1 + 1;
 constexpr size_t kNoAllocScratchBytes = align256(kOffScanTiles + kScanWords * sizeof(uint32_t));
 static_assert(kNoAllocScratchBytes == GMPM_NOALLOC_SCRATCH_BYTES, "keep include/gmpm.h in step");
 

@@ -24,8 +24,9 @@ constexpr int kScanTile = kScanThreads * kScanItems;
 inline int64_t scan_tiles(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
 
 // Working words of the binning's three scans (page flags, grid flags, cell
-// counts), one after the other: a status word per tile and the ticket.  They
-// are zero between binnings (the last kernel of a binning clears them).
+// counts), one after the other: a status word per tile and the ticket.  The
+// last word is set when a wait of any of them gave up.  They are zero between
+// binnings (the last kernel of a binning clears them).
 struct ScanScratch {
     uint32_t* words;
     int32_t count;
@@ -33,7 +34,7 @@ struct ScanScratch {
     int32_t* tile_sums;   // the batched scans' tile sums: one per tile of the longer of the key space and the cells, + 1
 };
 inline int64_t scan_scratch_words(int64_t key_space, int64_t ncell) {
-    return 2 * (scan_tiles(key_space) + 1) + scan_tiles(ncell) + 1;
+    return 2 * (scan_tiles(key_space) + 1) + scan_tiles(ncell) + 1 + 1;
 }
 inline ScanScratch scan_scratch(uint32_t* words, int64_t key_space, int64_t ncell, int32_t* tile_sums = nullptr) {
     const int32_t k = (int32_t)scan_tiles(key_space) + 1;
@@ -82,7 +83,9 @@ __device__ __forceinline__ int scan_take_tile(uint32_t* ticket) {
 }
 
 // Sum of the tiles before `tile`, whose own sum is `total`; every thread of the
-// CTA calls it.  `bad`: a wait gave up here or before (the sum is then 0).
+// CTA calls it.  `bad`: a wait gave up here or before (the sum is then 0).  A
+// tile after a bad one may still get its sum (it read the bad tile's own sum
+// and waited longer), so every bad tile reports, not only the last.
 __device__ __forceinline__ int32_t scan_look_back(uint32_t* status, int tile, int32_t total, bool& bad) {
     __shared__ int32_t s_prefix;
     __shared__ int s_bad;
