@@ -286,8 +286,8 @@ __device__ __forceinline__ void neo_hookean_fracture_from_svd(const MaterialDev<
     o.vol = V0 * det3(Fin);
 }
 
-// FP32 von Mises update for small strains, |F F^T - I| <= 0.1 (Frobenius; false
-// otherwise, and where the projected strain is larger).  The model is
+// FP32 von Mises update for small strains, |F F^T - I| <= 0.1 and det F > 0
+// (Frobenius; false otherwise, and where the projected strain is larger).  The model is
 // isotropic, so every quantity is a polynomial I, G, G^2 of G = F F^T - I, with
 // coefficients from G's invariants (Cayley-Hamilton reduces the higher powers):
 // the Hencky strain by the logarithm's series, the projected state by the
@@ -329,6 +329,8 @@ __device__ __forceinline__ bool small_strain_update(const MaterialDev<MR>& m, fl
     square(A, B);
     const float n2 = B[0] + B[1] + B[2];  // |G|^2
     if (!(n2 <= 0.01f)) return false;
+    // F F^T does not tell a reflection from a rotation; the SVD path does, and its stress is then not a number
+    if (!(det3(Fin) > 0.f)) return false;
     // eps = 1/2 log(I + G) = e0 I + e1 G + e2 G^2, with (p0, p1, p2) the coefficients of G^3, G^4, ...
     const float i1 = A[0] + A[1] + A[2], i2 = 0.5f * (i1 * i1 - n2), i3 = det(A);
     float e0 = 0.f, e1 = 0.5f, e2 = -0.25f;
