@@ -84,7 +84,7 @@ __device__ __forceinline__ void scan_gave_up(uint32_t* failed, Counters* cnt) {
 }
 // The page scan found pages and no wait gave up (n >= 1, so there are pages).
 __device__ __forceinline__ bool scans_done(const ScanScratch& scan, const Counters* cnt) {
-    return scan.words[scan.count - 1] == 0u && cnt->n_blocks > 0;
+    return (scan.words[scan.count - 1] == 0u) & (cnt->n_blocks > 0);  // both loads at once
 }
 
 // Ranks of the flagged keys in ascending order, with their list and count:
@@ -169,9 +169,9 @@ __device__ __forceinline__ void cell_scan_body(VB vb, int64_t ncell, int32_t* __
     if (clear0) zero_bytes_body(vb, clear0, key_space);
     if (clear1) zero_bytes_body(vb, clear1, key_space);
     uint32_t* words = scan.words + scan.cells;
-    // read once per CTA: a peer that gives up may set the failure word meanwhile
+    // read once per CTA (a peer that gives up may set the failure word meanwhile), beside thread 0's ticket
     __shared__ int64_t live;
-    if (threadIdx.x == 0) live = scans_done(scan, cnt) ? min(ncell, (int64_t)cnt->n_blocks * 64) : 0;
+    if (threadIdx.x == 32) live = scans_done(scan, cnt) ? min(ncell, (int64_t)cnt->n_blocks * 64) : 0;
     const int tile = scan_take_tile(words + (ncell + kScanTile - 1) / kScanTile);  // with a barrier
     const int64_t m = live;
     const int64_t base = (int64_t)tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
@@ -241,11 +241,12 @@ __device__ __forceinline__ void page_links_body(VB vb, const BinDev& bin, const 
     }
 }
 
-// Histogram of (page rank, cell) buckets with warp-aggregated atomics.
+// Histogram of (page rank, cell) buckets with warp-aggregated atomics.  done: the ranks are there (if not, nothing is
+// counted); used late, so that its loads travel beside the keys'.
 template <int kILP>
 __device__ __forceinline__ void bin_hist_body(VB vb, int64_t n, const uint32_t* __restrict__ keys,
                                               const int32_t* __restrict__ page_rank, int32_t* __restrict__ cell_count,
-                                              int nb_cap) {
+                                              int nb_cap, bool done) {
     const int64_t i0 = (int64_t)vb.b * kBinThreads * kILP + threadIdx.x;
     uint32_t key[kILP];
     int rank[kILP];
@@ -257,7 +258,7 @@ __device__ __forceinline__ void bin_hist_body(VB vb, int64_t n, const uint32_t* 
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int u = 0; u < kILP; ++u) {
-        const int bucket = rank[u] < nb_cap ? rank[u] * 64 + (int)(key[u] & 63) : -1;
+        const int bucket = done && rank[u] < nb_cap ? rank[u] * 64 + (int)(key[u] & 63) : -1;
         const unsigned peers = __match_any_sync(0xffffffffu, bucket);
         if (bucket >= 0 && lane == __ffs(peers) - 1) atomicAdd(&cell_count[bucket], __popc(peers));
     }
@@ -272,12 +273,12 @@ __host__ __device__ inline int bin_ctas(int64_t n, int ilp) {
 template <int kILP>
 __global__ void __launch_bounds__(kBinThreads) k_bin_hist_links(BinDev bin, ScanScratch scan, const Counters* cnt) {
     depend_on_previous();
-    if (!scans_done(scan, cnt)) return;
+    const bool done = scans_done(scan, cnt);
     const VB vb = own_blocks();
     const int hist = bin_ctas(bin.n, kILP);
     if (vb.b < hist)
-        bin_hist_body<kILP>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap);
-    else
+        bin_hist_body<kILP>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap, done);
+    else if (done)
         page_links_body(VB{vb.b - hist, vb.g - hist}, bin, cnt);
 }
 
@@ -288,7 +289,7 @@ __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_
                                                  const int32_t* __restrict__ page_rank,
                                                  const int32_t* __restrict__ cell_start, int32_t* __restrict__ fill,
                                                  int32_t* __restrict__ perm, uint32_t* __restrict__ keys_sorted,
-                                                 int nb_cap) {
+                                                 int nb_cap, bool done) {
     const int64_t i0 = (int64_t)vb.b * kBinThreads * kILP + threadIdx.x;
     uint32_t key[kILP];
     int bucket[kILP], start[kILP];
@@ -297,7 +298,7 @@ __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_
 #pragma unroll
     for (int u = 0; u < kILP; ++u) {
         const int r = i0 + (int64_t)u * kBinThreads < n ? page_rank[key[u] >> 6] : nb_cap;
-        bucket[u] = r < nb_cap ? r * 64 + (int)(key[u] & 63) : -1;
+        bucket[u] = done && r < nb_cap ? r * 64 + (int)(key[u] & 63) : -1;
     }
 #pragma unroll
     for (int u = 0; u < kILP; ++u) start[u] = kOffsets && bucket[u] >= 0 ? cell_start[bucket[u]] : 0;
@@ -320,12 +321,10 @@ __device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_
 template <int kILP>
 __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(BinDev bin, ScanScratch scan, Counters* cnt) {
     depend_on_previous();
-    if (!scans_done(scan, cnt)) {  // without starts the counts are no fill pointers; no pages for the kernels after
-        if (blockIdx.x == 0 && threadIdx.x == 0) cnt->n_blocks = cnt->n_grid_blocks = 0;
-        return;
-    }
+    const bool done = scans_done(scan, cnt);  // if not, the counts are no fill pointers: nothing is scattered
     bin_scatter_body<kILP, false>(own_blocks(), bin.n, bin.keys, bin.page_rank, nullptr, bin.cell_count, bin.perm,
-                                  bin.keys_sorted, bin.nb_cap);
+                                  bin.keys_sorted, bin.nb_cap, done);
+    if (!done && blockIdx.x == 0 && threadIdx.x == 0) cnt->n_blocks = cnt->n_grid_blocks = 0;  // for the kernels after
 }
 
 // Canonical in-cell order: ascending previous slot.  Each warp takes one page
@@ -711,9 +710,9 @@ __global__ void __launch_bounds__(kBinThreads) k_batch_hist(const SceneArgs<R>* 
                                                             const int32_t* __restrict__ start, int ns) {
     VB vb;
     const SceneArgs<R>& a = A[scene_of_block(start, ns, vb)];
-    if (a.cnt->n_blocks <= 0) return;  // no page has a flag (a binning before gave up): ranks and starts are not its own
+    const bool done = a.cnt->n_blocks > 0;  // else no page has a flag (a binning before gave up): ranks and starts are old
     const BinDev& bin = a.bin;
-    bin_hist_body<kBinILP>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap);
+    bin_hist_body<kBinILP>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_count, bin.nb_cap, done);
 }
 
 template <typename R>
@@ -721,10 +720,10 @@ __global__ void __launch_bounds__(kBinThreads) k_batch_scatter(const SceneArgs<R
                                                                const int32_t* __restrict__ start, int ns) {
     VB vb;
     const SceneArgs<R>& a = A[scene_of_block(start, ns, vb)];
-    if (a.cnt->n_blocks <= 0) return;
+    const bool done = a.cnt->n_blocks > 0;
     const BinDev& bin = a.bin;
     bin_scatter_body<kBinILP, true>(vb, bin.n, bin.keys, bin.page_rank, bin.cell_start, bin.cell_count, bin.perm, bin.keys_sorted,
-                     bin.nb_cap);
+                     bin.nb_cap, done);
 }
 
 template <typename R>
