@@ -328,8 +328,8 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(BinDev bin, ScanScr
 }
 
 // Canonical in-cell order: ascending previous slot.  Each warp takes one page
-// (8 pages per CTA in flight, so the page's few dependent global round trips
-// overlap across pages) and ranks every slot within its cell in shared memory
+// (up to 8 pages per CTA in flight, so the page's few dependent global round
+// trips overlap across pages) and ranks every slot within its cell in shared memory
 // (cells hold few particles).  A page above the warp's buffer is left to the
 // whole CTA, which ranks it in windows of whole cells after the warps'
 // pages; a single cell above the CTA buffer (thousands of particles in one
@@ -434,8 +434,8 @@ __device__ __forceinline__ void bin_canon_body(VB vb, const BinDev& bin, const S
     if (vb.b == 0)
         for (int q = threadIdx.x; q < scan.count; q += blockDim.x) scan.words[q] = 0u;
     if (nb <= 0) zero_bytes_body(vb, bin.cell_count, (int64_t)bin.nb_cap * 64 * 4);
-    for (int g = vb.b * kCanonWarps; g < nb; g += vb.g * kCanonWarps) {
-        const int b = g + warp;
+    for (int g = vb.b; g < nb; g += vb.g * kCanonWarps) {
+        const int b = g + warp * vb.g;
         int is_big = 0;
         if (b < nb) {
             for (int q = lane; q < 65; q += 32) cs[warp][q] = bin.cell_start[(int64_t)b * 64 + q];
@@ -490,7 +490,11 @@ __global__ void __launch_bounds__(32 * kCanonWarps) k_bin_canon(BinDev bin, Scan
     bin_canon_body(own_blocks(), bin, scan, cnt);
 }
 
-static int canon_ctas(int nb_cap, int sms) { return std::max(1, std::min((nb_cap + kCanonWarps - 1) / kCanonWarps, sms * 8)); }
+// About a CTA for each live page (the capacity is twice their number at creation), as far as they are resident at once,
+// and pages dealt out one per CTA before a second: pages above a warp's buffer take a whole CTA each.  (Eight neighbouring
+// pages per CTA left the work of dense scenes to a few CTAs, which a dependent launch also packs onto few SMs: binning of
+// 1M particles, 27 per cell 197 -> 56 us, 64 per cell 453 -> 100; 8 per cell 51 -> 46.)
+static int canon_ctas(int nb_cap, int sms) { return std::max(1, std::min((nb_cap + 1) / 2, sms * 8)); }
 
 // ---------------------------------------------------------------------------
 
@@ -575,7 +579,7 @@ void batch_scene_ctas(int64_t n, uint32_t key_space, int nb_cap, int ng_cap, int
     ctas[BM_LINKS] = cdiv((int64_t)std::max(nb_cap, ng_cap) * 8, 256);
     ctas[BM_ZERO_CELLS] = cdiv(ncell * 4, 4096);
     ctas[BM_CELL_TILES] = (int)scan_tiles(ncell);
-    ctas[BM_CANON] = canon_ctas(nb_cap, sms);
+    ctas[BM_CANON] = std::min(cdiv(nb_cap, kCanonWarps), sms * 8);
     ctas[BM_P2G] = real_bytes == 4 ? p2g_ctas<float>(nb_cap, sms) : p2g_ctas<double>(nb_cap, sms);
     ctas[BM_GRID] = std::max(1, std::min(ng_cap / 4 + 1, sms * 8));
     const int per_sm = real_bytes == 4 ? 2 : 1;  // G2P's resident CTAs per SM
