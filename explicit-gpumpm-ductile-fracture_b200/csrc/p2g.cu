@@ -271,8 +271,10 @@ __device__ __forceinline__ void set_lane_cell(LaneCell& L, uint32_t page, int ce
 }
 
 // Sums of a gather item (see make_item): three nodes of a window column, over
-// the cell columns that reach it.  A cell column's cells are added first, then
-// the columns along y, then (compensated) along x.  The upper half is the
+// the cell columns that reach it, x-major.  A cell column's cells are added
+// first, then the up to nine columns, compensated.  (Compensating along x only
+// took 1% off the kernel and lost what the sums of one cell column had over
+// those of a lane per stencil column.)  The upper half is the
 // mirror image: node 5 - z takes cell 3 - cz at stencil node 2 - k.
 constexpr int kNextY = 4 - 3 * 64, kNextX = 16 - 9 * 64;  // a node's sum in the next cell column along y, x
 __device__ __forceinline__ void gather_item(const P2* __restrict__ sums, uint32_t w, P2 sum[3]) {
@@ -285,18 +287,14 @@ __device__ __forceinline__ void gather_item(const P2* __restrict__ sums, uint32_
     for (int z = 0; z < 3; ++z) sum[z].x = sum[z].y = comp[z].x = comp[z].y = 0;
 #pragma unroll 1
     for (int i = 0; i < ni; ++i) {
-        P2 c0 = src[0], c1 = add2(src[sk], src[sc]), c2 = add2(add2(src[2 * sk], src[sk + sc]), src[2 * sc]);
         const P2* col = src;
 #pragma unroll 1
-        for (int j = 1; j < nj; ++j) {
+        for (int j = 0; j < nj; ++j) {
+            kahan_add2(sum[0], comp[0], col[0]);
+            kahan_add2(sum[1], comp[1], add2(col[sk], col[sc]));
+            kahan_add2(sum[2], comp[2], add2(add2(col[2 * sk], col[sk + sc]), col[2 * sc]));
             col += kNextY;
-            c0 = add2(c0, col[0]);
-            c1 = add2(c1, add2(col[sk], col[sc]));
-            c2 = add2(c2, add2(add2(col[2 * sk], col[sk + sc]), col[2 * sc]));
         }
-        kahan_add2(sum[0], comp[0], c0);
-        kahan_add2(sum[1], comp[1], c1);
-        kahan_add2(sum[2], comp[2], c2);
         src += kNextX;
     }
 }
