@@ -58,7 +58,7 @@ __device__ __forceinline__ void grid_body(VB vb, const SceneDev<R>* __restrict__
             const R im = R(1) / mass;
             R v[3] = {ch[CH_P0] * im + sc->gravity[0] * dt, ch[CH_P1] * im + sc->gravity[1] * dt,
                       ch[CH_P2] * im + sc->gravity[2] * dt};
-            R cnew = cgrid;
+            R cnew = cgrid, dc = R(0);
             if (sc->phase_field == GMPM_PHASE_FIELD_IMPLICIT) {
                 // the solve's vectors (ExplicitTimeIntegrator.cu:913-935): rhs sum_p V w (c/dt + M)
                 // (volP2G_APIC) as r with x0 = 0, Jacobi diagonal sum_p V w (FP M + 1/dt)
@@ -80,8 +80,16 @@ __device__ __forceinline__ void grid_body(VB vb, const SceneDev<R>* __restrict__
                 P.tag[i] = 1;
             } else if (sc->phase_field == GMPM_PHASE_FIELD_EXPLICIT) {
                 const R diagv = ch[CH_VW] / dt + Mob * ch[CH_VWFP];
-                const R rhs = ch[CH_VW] * (cgrid / dt + Mob) - Mob * ch[CH_KC];
-                if (diagv != R(0)) cnew = rhs / diagv;
+                if constexpr (sizeof(R) == 4) {
+                    // rhs / diagv - cgrid with cgrid's share taken out of rhs: the difference of two numbers near 1
+                    // left dc with their rounding (1e-7 a substep, mostly downwards, and damage only falls)
+                    if (diagv != R(0)) dc = Mob * (fmaf(-cgrid, ch[CH_VWFP], ch[CH_VW]) - ch[CH_KC]) / diagv;
+                    cnew = cgrid + dc;
+                } else {
+                    const R rhs = ch[CH_VW] * (cgrid / dt + Mob) - Mob * ch[CH_KC];
+                    if (diagv != R(0)) cnew = rhs / diagv;
+                    dc = cnew - cgrid;
+                }
             }
             int gx, gy, gz;
             page_coords(bin.grid_keys[g], gx, gy, gz);
@@ -120,7 +128,7 @@ __device__ __forceinline__ void grid_body(VB vb, const SceneDev<R>* __restrict__
             out[GC_V0] = v[0];
             out[GC_V1] = v[1];
             out[GC_V2] = v[2];
-            out[GC_DC] = cnew - cgrid;
+            out[GC_DC] = dc;
             out[GC_CN] = cnew;
         }
         if (sc->phase_field == GMPM_PHASE_FIELD_IMPLICIT && !(mass > R(0))) {
