@@ -99,6 +99,88 @@ __device__ __forceinline__ void p2g_barrier() {
     asm volatile("bar.sync 1, %0;\n" ::"n"(kP2GThreads) : "memory");
 }
 
+// Chunk sequence of one CTA: its pages b + k g (b, g: the CTA's index and the
+// CTA count of its scene's share of the launch).  A page of up to kP2GChunk
+// slots is one chunk.  A fuller page is cut into aligned runs of 32, 16, 8, ...
+// cells, each the largest that fits, whose particles several lanes share; a
+// single cell above kP2GChunk is cut by slots.  P2G of 1M particles with a lane
+// per cell of runs of kP2GChunk slots, and so: 16 per cell 167 -> 146 us, 32 per
+// cell 250 -> 169, 64 per cell 469 -> 221; 5,000 particles of 105k in one cell
+// 803 -> 187.  Every thread runs the same iterator.
+struct CellChunkIter {
+    int page, next, end;  // current page, next slot, page end
+    int cell;             // cell of the next slot (or an empty one before it)
+    int nbs, nbe;         // slot range of the following page (loaded one page ahead)
+    int stride;           // CTAs of the scene's share of the launch
+    __device__ void init(const BinDev& bin, int nb, VB vb) {
+        page = vb.b;
+        stride = vb.g;
+        next = end = cell = 0;
+        if (page < nb) {
+            next = bin.cell_start[(int64_t)page * 64];
+            end = bin.cell_start[(int64_t)page * 64 + 64];
+        }
+        preload(bin, nb);
+    }
+    __device__ void preload(const BinDev& bin, int nb) {
+        const int q = page + stride;
+        nbs = nbe = 0;
+        if (q < nb) {
+            nbs = bin.cell_start[(int64_t)q * 64];
+            nbe = bin.cell_start[(int64_t)q * 64 + 64];
+        }
+    }
+    // The next chunk of a page (start: its cells' starts) that is cut: its first slot, count and cells (as in step),
+    // and the cell after it.  Out of line, with few registers, for the sake of the pages that are not.
+    static __device__ __noinline__ int4 cut(const int32_t* start, int cell, int next) {
+        int n, cells;
+        do {
+            int stop[6];  // ends of the runs of 1, 2, 4, ... cells
+#pragma unroll
+            for (int q = 0; q < 6; ++q) stop[q] = start[min(cell + (1 << q), 64)];
+            int size = 1, e = min(stop[0], next + kP2GChunk);
+#pragma unroll
+            for (int q = 1; q < 6; ++q)
+                if ((cell & ((1 << q) - 1)) == 0 && stop[q] - next <= kP2GChunk) {
+                    size = 1 << q;
+                    e = stop[q];
+                }
+            n = e - next;
+            cells = size | cell << 8;
+            if (size > 1 || e == stop[0]) cell += size;
+        } while (n == 0);
+        return make_int4(next, n, cells, cell);
+    }
+    // Next chunk (page, first slot, count; 0 when done) and its cells: their number (a power of two), << 8 the
+    // first, kLastChunk: the last chunk of its page.
+    __device__ void step(const BinDev& bin, int nb, int& b, int& s0, int& n, int& cells) {
+        while (page < nb && next >= end) {
+            page += stride;
+            next = nbs;
+            end = nbe;
+            cell = 0;
+            if (page < nb) preload(bin, nb);
+        }
+        b = -1;
+        s0 = n = cells = 0;
+        if (page >= nb) return;
+        b = page;
+        s0 = next;
+        if (cell == 0 && end - next <= kP2GChunk) {
+            n = end - next;
+            cells = 64;
+        } else {
+            const int4 r = cut(bin.cell_start + (int64_t)page * 64, cell, next);
+            n = r.y;
+            cells = r.z;
+            cell = r.w;
+        }
+        next = s0 + n;
+        if (next >= end) cells |= kLastChunk;
+    }
+    static constexpr int kLastChunk = 1 << 16;
+};
+
 // What a lane keeps about its cell and the scene.
 struct LaneCell {
     R b[3];           // base node coordinates
@@ -139,13 +221,14 @@ __device__ __forceinline__ void add_terms(const P2 P[3], const P2 Q[3], const P2
         }
 }
 
-// A lane's particles [lo, hi): o holds their previous slots, w0 the first one staged.  Loading the next particle's words
-// ahead was slower (730 against 715 us at 8.4M particles): the moves it takes cost more than the latency.
-template <int N, typename F>
-__device__ __forceinline__ void sweep(const R* stage, const int32_t* o, int w0, int lo, int hi, const int (&plane)[N],
-                                      F add) {
+// A lane's particles lo, lo + step, ... below hi: o holds their previous slots, w0 the first one staged.  Loading the
+// next particle's words ahead was slower (730 against 715 us at 8.4M particles): the moves it takes cost more than the
+// latency.
+template <bool kStep, int N, typename F>
+__device__ __forceinline__ void sweep(const R* stage, const int32_t* o, int w0, int lo, int hi, int step,
+                                      const int (&plane)[N], F add) {
 #pragma unroll 1
-    for (int p = lo; p < hi; ++p) {
+    for (int p = lo; p < hi; p += kStep ? step : 1) {
         const R* s = stage + (o[p] - w0);
         R v[N];
 #pragma unroll
@@ -243,6 +326,30 @@ __device__ __forceinline__ void add_weights(const R (&v)[5], const LaneCell& L, 
                 one[q] += X1[i] * yz;
             }
         }
+}
+
+// Sums of `step` neighbouring lanes that share a cell (a power of two), in the
+// lane that writes them; the others write zeros, to cells without particles.
+template <typename T>
+__device__ __forceinline__ void share_sums(T acc[27], int step, bool writes);
+template <>
+__device__ __forceinline__ void share_sums(R acc[27], int step, bool writes) {
+#pragma unroll 1
+    for (int o = 1; o < step; o <<= 1)
+#pragma unroll
+        for (int q = 0; q < 27; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+#pragma unroll
+    for (int q = 0; q < 27; ++q) acc[q] = writes ? acc[q] : R(0);
+}
+template <>
+__device__ __forceinline__ void share_sums(P2 acc[27], int step, bool writes) {
+#pragma unroll 1
+    for (int o = 1; o < step; o <<= 1)
+#pragma unroll
+        for (int q = 0; q < 27; ++q)
+            acc[q] = add2(acc[q], pk(__shfl_xor_sync(0xffffffffu, acc[q].x, o), __shfl_xor_sync(0xffffffffu, acc[q].y, o)));
+#pragma unroll
+    for (int q = 0; q < 27; ++q) acc[q] = writes ? acc[q] : pk(R(0), R(0));
 }
 
 // Cell sums of a page, [slot][stencil node][cell] pairs: slots 0..2 are groups
@@ -387,6 +494,71 @@ constexpr size_t p2g_stage_bytes() {
 }
 static_assert(2 * sizeof(float) * kSlots * kSlotStride <= p2g_stage_bytes(), "cell sums fit the staged planes");
 
+// Cell sums of a chunk: this lane's particles lo, lo + step, ... below hi of its cell (L), summed into column `cell`.
+// Each group's sums stay in its own registers over the CTA's barrier, after which they overwrite the staged planes.
+// kShared: `step` neighbouring lanes share the cell, and one of them writes.
+template <bool kShared>
+__device__ __forceinline__ void cell_sums(const R* stage, P2* sums, const int32_t* o, int win, int group, int cell, int lo,
+                                          int hi, int step, bool writes, const LaneCell& L) {
+    P2 acc[27];
+#pragma unroll
+    for (int q = 0; q < 27; ++q) acc[q] = pk(R(0), R(0));
+    P2* out = sums + group * kSlotStride + cell;
+    if (group == 0)
+        sweep<kShared>(stage, o, win, lo, hi, step, kWordsXY, [&](auto& v) { add_momentum_xy(v, L, acc); });
+    else if (group == 1)
+        sweep<kShared>(stage, o, win, lo, hi, step, kWordsZQ, [&](auto& v) { add_momentum_z_flux(v, L, acc); });
+    else if (group == 2)
+        sweep<kShared>(stage, o, win, lo, hi, step, kWordsMC, [&](auto& v) { add_mass_damage(v, L, acc); });
+    if (group < 3) {
+        if (kShared) share_sums(acc, step, writes);
+        if (threadIdx.x == 0) bulk_store_wait_read();  // the previous tile has left shared memory
+        p2g_barrier();
+#pragma unroll
+        for (int q = 0; q < 27; ++q) out[q * 64] = acc[q];
+    } else {
+        R one[27];
+#pragma unroll
+        for (int q = 0; q < 27; ++q) one[q] = R(0);
+        sweep<kShared>(stage, o, win, lo, hi, step, kWordsV, [&](auto& v) { add_weights(v, L, acc, one); });
+        if (kShared) {
+            share_sums(acc, step, writes);
+            share_sums(one, step, writes);
+        }
+        p2g_barrier();
+#pragma unroll
+        for (int q = 0; q < 27; ++q) {
+            out[q * 64] = acc[q];
+            out[kSlotStride + q * 64] = pk(one[q], R(0));
+        }
+    }
+}
+
+// Cell sums of a chunk of part of a page's cells: a group's 64 lanes share them, up to 32 lanes (of one warp) each.  Out
+// of line and with loops of its own, for the sake of whole pages (P2G of 1M particles, 8 per cell: 131.6 us; 132.5 with
+// this inlined, 142 with one loop for both forms).
+__device__ __noinline__ void shared_cell_sums(const R* stage, P2* sums, const int32_t* o, const int32_t* cs, uint32_t page,
+                                              int win, int c0, int n0, int cells, int group, bool lighter, R dx, R inv_dx,
+                                              R kD, R kS) {
+    const int nc = cells & 127, ca = (cells >> 8) & 63, vl = (threadIdx.x & 31) + (lighter ? 32 : 0);
+    const int step = min(64 / nc, 32), c = vl / step, sub = vl & (step - 1);
+    int cell = min(ca + c, ca + nc - 1);
+    LaneCell L;
+    L.dx = dx;
+    L.inv_dx = inv_dx;
+    L.kD = kD;
+    L.kS = kS;
+    set_lane_cell(L, page, cell);
+    const int hi = min(cs[cell + 1], c0 + n0) - c0;
+    const int lo = c < nc ? max(cs[cell], c0) - c0 + sub : hi;
+    const bool writes = c < nc && sub == 0;
+    if (!writes) {  // the cell it writes zeros to: as many are without particles as lanes do not write
+        const int j = c < nc ? vl - c - 1 : vl - nc;
+        cell = j < ca ? j : j + nc;
+    }
+    cell_sums<true>(stage, sums, o, win, group, cell, lo, hi, step, writes, L);
+}
+
 __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ sc, const PState<R>& st,
                                          const PAux<R>& aux, const BinDev& bin, R* __restrict__ tile,
                                          Counters* __restrict__ cnt) {
@@ -409,11 +581,11 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
     L.kS = -sc->dt * sc->inv_dx;
 
     // prologue: descriptors of chunks 0 and 1, meta of chunk 0
-    ChunkIter<kP2GChunk> it;
+    CellChunkIter it;
     it.init(bin, nb, vb);
-    int b0, c0, n0, last0, b1, c1, n1, last1;
-    it.step(bin, nb, b0, c0, n0, last0);
-    it.step(bin, nb, b1, c1, n1, last1);
+    int b0, c0, n0, cells0, b1, c1, n1, cells1;
+    it.step(bin, nb, b0, c0, n0, cells0);
+    it.step(bin, nb, b1, c1, n1, cells1);
     if (t == 0) {
         S.abort = 0;
         mbar_init(&S.bar, kP2GThreads / 32);
@@ -464,37 +636,11 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
         if (outside) sort_staged(S.plane, S.o[m], stage, n0, w0, len);
         const int win = (int)w0;
 
-        // Cell sums.  Each group's sums stay in its own registers over the CTA's barrier, after which they
-        // overwrite the staged planes.
-        {
-            P2 acc[27];
-#pragma unroll
-            for (int q = 0; q < 27; ++q) acc[q] = pk(R(0), R(0));
-            P2* out = sums + group * kSlotStride + cell;
-            if (group == 0)
-                sweep(stage, S.o[m], win, lo, hi, kWordsXY, [&](auto& v) { add_momentum_xy(v, L, acc); });
-            else if (group == 1)
-                sweep(stage, S.o[m], win, lo, hi, kWordsZQ, [&](auto& v) { add_momentum_z_flux(v, L, acc); });
-            else if (group == 2)
-                sweep(stage, S.o[m], win, lo, hi, kWordsMC, [&](auto& v) { add_mass_damage(v, L, acc); });
-            if (group < 3) {
-                if (t == 0) bulk_store_wait_read();  // the previous tile has left shared memory
-                p2g_barrier();
-#pragma unroll
-                for (int q = 0; q < 27; ++q) out[q * 64] = acc[q];
-            } else {
-                R one[27];
-#pragma unroll
-                for (int q = 0; q < 27; ++q) one[q] = R(0);
-                sweep(stage, S.o[m], win, lo, hi, kWordsV, [&](auto& v) { add_weights(v, L, acc, one); });
-                p2g_barrier();
-#pragma unroll
-                for (int q = 0; q < 27; ++q) {
-                    out[q * 64] = acc[q];
-                    out[kSlotStride + q * 64] = pk(one[q], R(0));
-                }
-            }
-        }
+        if (cells0 & 64)
+            cell_sums<false>(stage, sums, S.o[m], win, group, cell, lo, hi, 1, true, L);
+        else
+            shared_cell_sums(stage, sums, S.o[m], S.cs[m], S.bkey[m], win, c0, n0, cells0, group, lighter, L.dx, L.inv_dx,
+                             L.kD, L.kS);
         __syncthreads();
         // Gather: window column (a, b), slot and half of the column's six nodes per item.  A node sums its
         // cell columns (cx, cy) = (a - i, b - j) in ascending order (compensated), each column's cells
@@ -522,10 +668,10 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
                 }
             }
         }
-        if (last0) done = b0;
-        first = last0 != 0;
-        b0 = b1; c0 = c1; n0 = n1; last0 = last1;
-        it.step(bin, nb, b1, c1, n1, last1);
+        first = (cells0 & CellChunkIter::kLastChunk) != 0;
+        if (first) done = b0;
+        b0 = b1; c0 = c1; n0 = n1; cells0 = cells1;
+        it.step(bin, nb, b1, c1, n1, cells1);
     }
     cp_async_wait_all();
     if (t == 0) bulk_store_wait();
