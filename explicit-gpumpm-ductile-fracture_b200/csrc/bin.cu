@@ -93,10 +93,10 @@ __device__ __forceinline__ bool scans_done(const ScanScratch& scan, const Counte
 // (supplementAdjacentPages, Transformer_kernal.cu:70-96).  words: the scan's
 // status words and, after them, its ticket.  Ranks of keys without a flag are
 // left as they are; no reader looks at them.  failed: set where a wait gave up.
-__device__ __forceinline__ void page_scan_body(uint32_t key_space, const uint8_t* __restrict__ flag,
-                                               int32_t* __restrict__ rank, uint32_t* __restrict__ list, int cap,
-                                               int32_t* __restrict__ total, uint8_t* __restrict__ grid_flag,
-                                               uint32_t* __restrict__ words, uint32_t* failed, Counters* cnt) {
+__device__ __forceinline__ void page_scan_body(uint32_t key_space, const uint8_t* flag,
+                                               int32_t* rank, uint32_t* list, int cap,
+                                               int32_t* total, uint8_t* grid_flag,
+                                               uint32_t* words, uint32_t* failed, Counters* cnt) {
     const int ntiles = (int)((key_space + kScanTile - 1) / kScanTile);
     const int tile = scan_take_tile(words + ntiles);
     if (tile >= ntiles) return;
@@ -145,9 +145,9 @@ __device__ __forceinline__ void page_scan_body(uint32_t key_space, const uint8_t
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-    k_page_scan(uint32_t key_space, const uint8_t* __restrict__ flag, int32_t* __restrict__ rank,
-                uint32_t* __restrict__ list, int cap, int32_t* __restrict__ total, uint8_t* __restrict__ grid_flag,
-                uint32_t* __restrict__ words, uint32_t* failed, Counters* cnt) {
+    k_page_scan(uint32_t key_space, const uint8_t* flag, int32_t* rank,
+                uint32_t* list, int cap, int32_t* total, uint8_t* grid_flag,
+                uint32_t* words, uint32_t* failed, Counters* cnt) {
     depend_on_previous();
     page_scan_body(key_space, flag, rank, list, cap, total, grid_flag, words, failed, cnt);
 }
@@ -163,8 +163,8 @@ __device__ __forceinline__ void zero_bytes_body(VB vb, void* p, int64_t bytes) {
 // total after them.  The starts also replace the counts, as the scatter's fill
 // pointers.  clear: flags whose last use in the binning was the page links,
 // cleared here for the next one (or null).
-__device__ __forceinline__ void cell_scan_body(VB vb, int64_t ncell, int32_t* __restrict__ count,
-                                               int32_t* __restrict__ start, const ScanScratch& scan,
+__device__ __forceinline__ void cell_scan_body(VB vb, int64_t ncell, int32_t* count,
+                                               int32_t* start, const ScanScratch& scan,
                                                uint8_t* clear0, uint8_t* clear1, uint32_t key_space, Counters* cnt) {
     if (clear0) zero_bytes_body(vb, clear0, key_space);
     if (clear1) zero_bytes_body(vb, clear1, key_space);
@@ -205,7 +205,7 @@ __device__ __forceinline__ void cell_scan_body(VB vb, int64_t ncell, int32_t* __
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-    k_cell_scan(int64_t ncell, int32_t* __restrict__ count, int32_t* __restrict__ start, ScanScratch scan,
+    k_cell_scan(int64_t ncell, int32_t* count, int32_t* start, ScanScratch scan,
                 uint8_t* clear0, uint8_t* clear1, uint32_t key_space, Counters* cnt) {
     depend_on_previous();
     cell_scan_body(own_blocks(), ncell, count, start, scan, clear0, clear1, key_space, cnt);
@@ -244,8 +244,8 @@ __device__ __forceinline__ void page_links_body(VB vb, const BinDev& bin, const 
 // Histogram of (page rank, cell) buckets with warp-aggregated atomics.  done: the ranks are there (if not, nothing is
 // counted); used late, so that its loads travel beside the keys'.
 template <int kILP>
-__device__ __forceinline__ void bin_hist_body(VB vb, int64_t n, const uint32_t* __restrict__ keys,
-                                              const int32_t* __restrict__ page_rank, int32_t* __restrict__ cell_count,
+__device__ __forceinline__ void bin_hist_body(VB vb, int64_t n, const uint32_t* keys,
+                                              const int32_t* page_rank, int32_t* cell_count,
                                               int nb_cap, bool done) {
     const int64_t i0 = (int64_t)vb.b * kBinThreads * kILP + threadIdx.x;
     uint32_t key[kILP];
@@ -285,10 +285,10 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_hist_links(BinDev bin, Scan
 // Scatter slots; lanes of one warp with the same bucket keep their order.  fill: the cells' fill pointers, or
 // (kOffsets) fill counts beside the cells' starts.
 template <int kILP, bool kOffsets>
-__device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_t* __restrict__ keys,
-                                                 const int32_t* __restrict__ page_rank,
-                                                 const int32_t* __restrict__ cell_start, int32_t* __restrict__ fill,
-                                                 int32_t* __restrict__ perm, uint32_t* __restrict__ keys_sorted,
+__device__ __forceinline__ void bin_scatter_body(VB vb, int64_t n, const uint32_t* keys,
+                                                 const int32_t* page_rank,
+                                                 const int32_t* cell_start, int32_t* fill,
+                                                 int32_t* perm, uint32_t* keys_sorted,
                                                  int nb_cap, bool done) {
     const int64_t i0 = (int64_t)vb.b * kBinThreads * kILP + threadIdx.x;
     uint32_t key[kILP];

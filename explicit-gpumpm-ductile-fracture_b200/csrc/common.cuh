@@ -83,6 +83,14 @@ struct SceneDev {
     double cfl_dx;          // cfl_number * dx
 };
 
+// The time step, the one value of the scene block that a kernel writes (the
+// clock, in adaptive mode): read where it stands, also through a pointer that
+// promises a block without writers (launch.cuh).
+template <typename Real>
+__device__ __forceinline__ Real scene_dt(const SceneDev<Real>* sc) {
+    return *const_cast<const volatile Real*>(&sc->dt);
+}
+
 // Counters and flags living in device memory (written by kernels, read by host on demand).
 struct Counters {
     int n_blocks;

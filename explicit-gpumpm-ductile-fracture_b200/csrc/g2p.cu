@@ -378,7 +378,7 @@ __device__ __forceinline__ void decode_pages(G2PShared<R>& S, int seq0, int np) 
 // numbers in [wseq0, wseq1) (the pages not staged by the previous unit).
 template <typename R>
 __device__ __forceinline__ void issue_data(G2PShared<R>& S, int m, int buf, int n, int wseq0, int wseq1,
-                                           const PState<R>& in, const R* __restrict__ nodes) {
+                                           const PState<R>& in, const R* nodes) {
     const int t = threadIdx.x;
     if (t < n) {
         const int o = S.o[m][t];
@@ -419,12 +419,12 @@ template <typename R, bool kAnyModel, bool kFallback>
 __device__ __forceinline__ void g2p_body(VB vb, const SceneDev<R>* __restrict__ sc,
                                          const SceneDev<double>* __restrict__ sc64, const PState<R>& in,
                                          const PState<R>& out, const PAux<R>& aux, const BinDev& bin,
-                                         const R* __restrict__ nodes, Counters* cnt) {
+                                         const R* nodes, Counters* cnt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     G2PShared<R>& S = *reinterpret_cast<G2PShared<R>*>(smem_raw);
     const int t = threadIdx.x;
     const int nb = min(cnt->n_blocks, bin.nb_cap);
-    const R dx = sc->dx, inv_dx = sc->inv_dx, dt = sc->dt, V0 = sc->V0;
+    const R dx = sc->dx, inv_dx = sc->inv_dx, dt = scene_dt(sc), V0 = sc->V0;
     const bool fallback = kFallback && sc->fp64_svd_fallback && sc64 != nullptr;
     const R ratio = sc->svd_fallback_ratio;
     unsigned int flags = 0;
@@ -621,7 +621,7 @@ __device__ __forceinline__ void g2p_body(VB vb, const SceneDev<R>* __restrict__ 
 template <typename R, bool kAnyModel, bool kFallback>
 __global__ void __launch_bounds__(kG2PUnit, sizeof(R) == 4 ? kG2PMinBlocks : 1)
     k_g2p(const SceneDev<R>* __restrict__ sc, const SceneDev<double>* __restrict__ sc64, PState<R> in,
-          PState<R> out, PAux<R> aux, BinDev bin, const R* __restrict__ nodes, Counters* cnt) {
+          PState<R> out, PAux<R> aux, BinDev bin, const R* nodes, Counters* cnt) {
     depend_on_previous();
     g2p_body<R, kAnyModel, kFallback>(own_blocks(), sc, sc64, in, out, aux, bin, nodes, cnt);
 }

@@ -22,9 +22,9 @@ namespace gmpm {
 constexpr int kGridThreads = 256;  // 4 grid pages per CTA
 
 template <typename R>
-__device__ __forceinline__ void grid_body(VB vb, const SceneDev<R>* __restrict__ sc, const BinDev& bin,
-                                          const R* __restrict__ tile, R* __restrict__ nodes,
-                                          double* __restrict__ diag, const PcgDev& pcg, Counters* cnt) {
+__device__ __forceinline__ void grid_body(VB vb, const SceneDev<R>* sc, const BinDev& bin,
+                                          const R* tile, R* nodes,
+                                          double* diag, const PcgDev& pcg, Counters* cnt) {
     const int ng = min(cnt->n_grid_blocks, bin.ng_cap);
     const int node = threadIdx.x & 63;
     const int ci = node >> 4, cj = (node >> 2) & 3, ck = node & 3;
@@ -158,8 +158,8 @@ __device__ __forceinline__ void grid_body(VB vb, const SceneDev<R>* __restrict__
 
 template <typename R>
 __global__ void __launch_bounds__(kGridThreads)
-    k_grid(const SceneDev<R>* __restrict__ sc, BinDev bin, const R* __restrict__ tile, R* __restrict__ nodes,
-           double* __restrict__ diag, PcgDev pcg, Counters* cnt) {
+    k_grid(const SceneDev<R>* sc, BinDev bin, const R* tile, R* nodes,
+           double* diag, PcgDev pcg, Counters* cnt) {
     depend_on_previous();
     grid_body<R>(own_blocks(), sc, bin, tile, nodes, diag, pcg, cnt);
 }

@@ -559,9 +559,9 @@ __device__ __noinline__ void shared_cell_sums(const R* stage, P2* sums, const in
     cell_sums<true>(stage, sums, o, win, group, cell, lo, hi, step, writes, L);
 }
 
-__device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ sc, const PState<R>& st,
-                                         const PAux<R>& aux, const BinDev& bin, R* __restrict__ tile,
-                                         Counters* __restrict__ cnt) {
+__device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* sc, const PState<R>& st,
+                                         const PAux<R>& aux, const BinDev& bin, R* tile,
+                                         Counters* cnt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* stage = reinterpret_cast<R*>(smem_raw);   // [kRawWords][WS] raw planes
     P2* sums = reinterpret_cast<P2*>(smem_raw);  // the page's cell sums, once the planes are read
@@ -687,8 +687,8 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
 }
 
 __global__ void __launch_bounds__(kP2GThreads, kCtasPerSm)
-    k_p2g(const SceneDev<R>* __restrict__ sc, PState<R> st, PAux<R> aux, BinDev bin, R* __restrict__ tile,
-            Counters* __restrict__ cnt, double* __restrict__ diag) {
+    k_p2g(const SceneDev<R>* sc, PState<R> st, PAux<R> aux, BinDev bin, R* tile,
+            Counters* cnt, double* diag) {
     depend_on_previous();
     // the sums that the grid stage adds to
     if (blockIdx.x == 0 && threadIdx.x < 4) diag[threadIdx.x] = 0.0;

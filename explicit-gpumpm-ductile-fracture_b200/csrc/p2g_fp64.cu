@@ -88,7 +88,7 @@ __device__ __forceinline__ void bspline1d(R xp, R inv_dx, R* w, R* g) {
 }
 
 // Build the particle's record from its raw words.
-__device__ __forceinline__ void build_record(const SceneDev<R>* __restrict__ sc, const int base[3], const R* raw,
+__device__ __forceinline__ void build_record(const SceneDev<R>* sc, const int base[3], const R* raw,
                                              R* rec) {
     const R dx = sc->dx, inv_dx = sc->inv_dx, dt = sc->dt, Dinv = sc->Dinv;
     R xp[3];
@@ -258,9 +258,9 @@ constexpr size_t p2g_stage_bytes() {
     return sizeof(R) * (size_t)kRawWords * Staging::WS;
 }
 
-__device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ sc, const PState<R>& st,
-                                         const PAux<R>& aux, const BinDev& bin, R* __restrict__ tile,
-                                         Counters* __restrict__ cnt) {
+__device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* sc, const PState<R>& st,
+                                         const PAux<R>& aux, const BinDev& bin, R* tile,
+                                         Counters* cnt) {
     constexpr int W = Staging::W, WS = Staging::WS;
     static_assert(sizeof(R) * kP2GChannels * kFlushChStride <= p2g_rec_bytes(), "column sums fit the record buffer");
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -458,8 +458,8 @@ __device__ __forceinline__ void p2g_body(VB vb, const SceneDev<R>* __restrict__ 
 }
 
 __global__ void __launch_bounds__(kP2GThreads, 1)
-    k_p2g64(const SceneDev<R>* __restrict__ sc, PState<R> st, PAux<R> aux, BinDev bin, R* __restrict__ tile,
-            Counters* __restrict__ cnt, double* __restrict__ diag) {
+    k_p2g64(const SceneDev<R>* sc, PState<R> st, PAux<R> aux, BinDev bin, R* tile,
+            Counters* cnt, double* diag) {
     depend_on_previous();
     // the sums that the grid stage adds to
     if (blockIdx.x == 0 && threadIdx.x < 4) diag[threadIdx.x] = 0.0;

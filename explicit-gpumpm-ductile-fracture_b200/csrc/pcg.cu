@@ -104,8 +104,8 @@ __device__ double combine_partials(const double* part, int n, bool use_max, doub
 
 // partial sums of a[i] b[i] over runs of 128 entries
 __global__ void __launch_bounds__(kPcgBlock)
-    k_pcg_dot(const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ part, BinDev bin,
-              const Counters* __restrict__ cnt) {
+    k_pcg_dot(const double* a, const double* b, double* part, BinDev bin,
+              const Counters* cnt) {
     depend_on_previous();
     __shared__ double sh[32];
     const int N = pcg_entries(cnt, bin);
@@ -137,8 +137,8 @@ __global__ void __launch_bounds__(kPcgScalarThreads)
 // one CTA per particle page with the page's 6x6x6 window of s staged.
 template <typename R>
 __global__ void __launch_bounds__(kPcgColThreads)
-    k_pcg_col(const SceneDev<R>* __restrict__ sc, PState<R> st, PAux<R> aux, BinDev bin, PcgDev P,
-              const Counters* __restrict__ cnt) {
+    k_pcg_col(const SceneDev<R>* sc, PState<R> st, PAux<R> aux, BinDev bin, PcgDev P,
+              const Counters* cnt) {
     depend_on_previous();
     if (P.scal->done) return;
     __shared__ double win[kWindowNodes];
@@ -258,8 +258,8 @@ __device__ __forceinline__ void kx_cell(const double* __restrict__ recs, const i
 // are bitwise reproducible.
 template <typename R>
 __global__ void __launch_bounds__(kPcgKxThreads, 4)
-    k_pcg_kx(const SceneDev<R>* __restrict__ sc, PState<R> st, BinDev bin, PcgDev P, double* __restrict__ tile,
-             const Counters* __restrict__ cnt) {
+    k_pcg_kx(const SceneDev<R>* sc, PState<R> st, BinDev bin, PcgDev P, double* tile,
+             const Counters* cnt) {
     depend_on_previous();
     if (P.scal->done) return;
     __shared__ double recs[kPcgKxChunk * kKxRec];  // staged particles; the column sums at a page's end
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kPcgKxThreads, 4)
 // q = D s + M K s on tagged nodes (K s: the 8 overlapping page tiles in slot
 // order); partial sums of s . q
 __global__ void __launch_bounds__(kPcgBlock)
-    k_pcg_q(BinDev bin, PcgDev P, const double* __restrict__ tile, const Counters* __restrict__ cnt,
+    k_pcg_q(BinDev bin, PcgDev P, const double* tile, const Counters* cnt,
             double mobility) {
     depend_on_previous();
     if (P.scal->done) return;
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kPcgBlock)
 }
 
 __global__ void __launch_bounds__(kPcgScalarThreads)
-    k_pcg_alpha(PcgDev P, BinDev bin, const Counters* __restrict__ cnt, int max_combine) {
+    k_pcg_alpha(PcgDev P, BinDev bin, const Counters* cnt, int max_combine) {
     depend_on_previous();
     if (P.scal->done) return;
     __shared__ double sh[32];
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kPcgScalarThreads)
 // x += alpha s, r -= alpha q, mr = r / D (precondition_subd) on tagged nodes;
 // partial max r^2 and partial sums of r . mr
 __global__ void __launch_bounds__(kPcgBlock)
-    k_pcg_update(BinDev bin, PcgDev P, const Counters* __restrict__ cnt) {
+    k_pcg_update(BinDev bin, PcgDev P, const Counters* cnt) {
     depend_on_previous();
     if (P.scal->done) return;
     __shared__ double sh[32];
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kPcgBlock)
 
 // residual norm, convergence, rho and the direction update rate
 __global__ void __launch_bounds__(kPcgScalarThreads)
-    k_pcg_rho(PcgDev P, BinDev bin, const Counters* __restrict__ cnt, int max_combine, double tol) {
+    k_pcg_rho(PcgDev P, BinDev bin, const Counters* cnt, int max_combine, double tol) {
     depend_on_previous();
     if (P.scal->done) return;
     __shared__ double sh[32];
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kPcgScalarThreads)
 }
 
 // s = s rate + mr on tagged nodes (cal_grid_r_vad_kernal)
-__global__ void __launch_bounds__(kPcgBlock) k_pcg_sdir(BinDev bin, PcgDev P, const Counters* __restrict__ cnt) {
+__global__ void __launch_bounds__(kPcgBlock) k_pcg_sdir(BinDev bin, PcgDev P, const Counters* cnt) {
     depend_on_previous();
     if (P.scal->done) return;
     const int N = pcg_entries(cnt, bin);
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kPcgBlock) k_pcg_sdir(BinDev bin, PcgDev P, co
 // dc = x - c_grid and c_new = x on tagged nodes (update_grid_phase, :632-642);
 // x = 1e20 everywhere after a breakdown (rho_old == 0)
 template <typename R>
-__global__ void k_pcg_finish(BinDev bin, PcgDev P, R* __restrict__ nodes, Counters* cnt) {
+__global__ void k_pcg_finish(BinDev bin, PcgDev P, R* nodes, Counters* cnt) {
     depend_on_previous();
     const int N = pcg_entries(cnt, bin);
     const bool blow = P.scal->blowup != 0;
