@@ -248,7 +248,7 @@ def run_ours(args, pkg, rank: int, local_rank: int, world: int, dist):
         what += ", implicit phase field (Jacobi-PCG, tol 1e-6, <= 100 iterations)"
     if getattr(args, "atomic_p2g", False):
         sp.desc.deterministic = 0
-        what += ", P2G node sums with shared-memory atomics (not bitwise reproducible)"
+        what += ", deterministic = 0 (the same fixed-order P2G)"
     t0 = time.perf_counter()
     scene = sp.build(ctx)
     build_s = time.perf_counter() - t0
@@ -514,7 +514,7 @@ def main():
     ap.add_argument("--reference-sample", action="store_true",
                     help="reference arm: time the bounded CPU sample instead of the whole workload")
     ap.add_argument("--atomic-p2g", action="store_true",
-                    help="P2G's fast mode (shared-memory atomics) instead of the fixed-order, reproducible sums")
+                    help="scenes with deterministic = 0, which run the same fixed-order P2G (there is no other)")
     args = ap.parse_args()
     if args.warmup < 3:
         args.warmup = 3
@@ -617,7 +617,7 @@ def main():
             steps=args.steps, warmup=args.warmup, ms_per_step=res["ms_max"] / args.steps, higher_is_better=True,
             scaling="weak", vs_baseline=None, dtype="f32", data="synthetic",
             config=dict(workload=res["what"], particles_per_gpu=sp.n, precision="fp32",
-                        deterministic_p2g=not args.atomic_p2g,
+                        deterministic_p2g=True,
                         parallelism=f"replicas x{world}" if world > 1 else "single scene",
                         l2="resident state larger than L2 (no flush needed)"),
             roofline=dict(bound="hbm", kernel=res["dom"], achieved=k["achieved_gbs"], peak=res["peaks"]["hbm_gbs"],

@@ -325,7 +325,7 @@ struct Scene : SceneBase {
     LaunchCfg cfg() const {
         int other = 0;
         for (int m = 0; m < desc.n_materials; ++m) other |= desc.materials[m].energy_model != GMPM_ENERGY_VON_MISES_FRACTURE;
-        return LaunchCfg{share_ > 0 ? std::min(share_, ctx->num_sms) : ctx->num_sms, desc.deterministic,
+        return LaunchCfg{share_ > 0 ? std::min(share_, ctx->num_sms) : ctx->num_sms,
                          desc.pcg_max_combine, desc.materials[0].mobility, desc.pcg_tolerance, other};
     }
     bool implicit_pf() const { return desc.phase_field == GMPM_PHASE_FIELD_IMPLICIT; }
@@ -630,7 +630,7 @@ struct Scene : SceneBase {
     int batch_kind() const override {
         if (implicit_pf()) return -1;
         const LaunchCfg lc = cfg();
-        return (sizeof(R) == 8 ? 8 : 0) | (desc.deterministic ? 4 : 0) | (lc.other_models ? 2 : 0) |
+        return (sizeof(R) == 8 ? 8 : 0) | (lc.other_models ? 2 : 0) |
                (desc.precision == GMPM_PRECISION_FP32_FP64SVD ? 1 : 0);
     }
     void batch_args(int c, void* out) const override {

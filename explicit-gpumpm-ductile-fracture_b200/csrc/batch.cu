@@ -3,7 +3,7 @@
 // uneven scenes, each with its own SPGrid, advances by one CUDA graph launch
 // per substep.
 //
-// Scene table: the scenes whose kernels are of one kind (precision, P2G mode,
+// Scene table: the scenes whose kernels are of one kind (precision,
 // energy models, FP64 fallback) form a group, and the group's substep is one
 // launch per stage over all its scenes (launch_batch_*, kernels.h): a device
 // array of the scenes' buffers and, per stage, each scene's range of CTAs.
@@ -232,7 +232,6 @@ struct Batch {
                 g.plan.total[k] = totals[k];
             }
             g.plan.n_scenes = m;
-            g.plan.deterministic = (g.kind & 4) != 0;
             g.plan.other_models = (g.kind & 2) != 0;
             g.plan.fallback = (g.kind & 1) != 0;
             // on the batch's own stream: the copies wait for nothing else on the device

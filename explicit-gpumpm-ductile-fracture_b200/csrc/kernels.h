@@ -44,7 +44,6 @@ struct GridDev {
 
 struct LaunchCfg {
     int num_sms;
-    int deterministic;
     int pcg_max_combine;   // implicit phase field settings
     double pcg_mobility;
     double pcg_tolerance;
@@ -128,8 +127,7 @@ cudaError_t launch_pack_field(const PState<R>& st, const PAux<R>& aux, int field
                               void* out, cudaStream_t stream);
 
 // ---- batched launches: one launch per stage over many scenes ------------------
-// A batch of scenes of one kind (precision, P2G mode, energy models, FP64
-// fallback) advances with one launch per stage of the substep.  Every stage
+// A batch of scenes of one kind (precision, energy models, FP64 fallback) advances with one launch per stage of the substep.  Every stage
 // splits its launch into per-scene CTA ranges (BatchPlan); a CTA finds its
 // scene by a search over its stage's range starts and runs the stage's body
 // for that scene with its place in the scene's range (VB, common.cuh).
@@ -188,7 +186,6 @@ struct BatchPlan {
     int n_scenes;
     const int32_t* start[kBatchMaps];  // device
     int total[kBatchMaps];             // CTAs of each launch
-    int deterministic;                 // P2G's fixed-order mode
     int other_models;                  // a material uses an energy model other than von Mises
     int fallback;                      // FP32 with the FP64 SVD fallback
 };

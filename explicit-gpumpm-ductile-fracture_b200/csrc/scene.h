@@ -57,7 +57,7 @@ struct SceneBase {
     virtual void set_sm_share(int sms) = 0;
     virtual int sm_share() const = 0;
     // One launch per stage over many scenes (kernels.h, BatchPlan): the kind of
-    // the scene's kernels (precision, P2G mode, energy models, FP64 fallback;
+    // the scene's kernels (precision, energy models, FP64 fallback;
     // -1 if the scene cannot join, as with the implicit phase field), its
     // buffers for a parity as a SceneArgs<R> (into out), and the sizes that
     // set its CTA ranges.
