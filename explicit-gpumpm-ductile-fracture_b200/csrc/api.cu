@@ -269,7 +269,7 @@ struct Scene : SceneBase {
     // positions (set by a key pass or by the G2P that wrote them), so the next
     // binning skips its key pass
     bool keys_fresh = false;
-    bool grid_dirty = false;  // the last binning was batched and left its grid flags set
+    bool bin_dirty = false;  // a binning's launches failed, so its working words may not be zero
     int64_t launches = 0;  // kernels launched by this scene
     uint64_t uid_ = g_scene_uid++;
     int share_ = 0;        // SMs the launch shapes are sized for (0: all)
@@ -542,9 +542,16 @@ struct Scene : SceneBase {
         return GMPM_OK;
     }
 
+    cudaError_t launch_bin(cudaStream_t s, int c, int num_sms, bool keys_ready) {
+        const bool reset = bin_dirty;
+        bin_dirty = true;
+        const cudaError_t e = launch_binning<R>(d_sc, st[c], bin, scan, d_cnt, num_sms, s, keys_ready, reset);
+        if (e == cudaSuccess) bin_dirty = false;
+        return e;
+    }
+
     gmpm_status do_bin(cudaStream_t s) {
-        GMPM_TRY(launch_binning<R>(d_sc, st[cur], bin, scan, d_cnt, cfg().num_sms, s, false, grid_dirty));
-        grid_dirty = false;
+        GMPM_TRY(launch_bin(s, cur, cfg().num_sms, false));
         binned = true;
         keys_fresh = true;
         return GMPM_OK;
@@ -560,7 +567,7 @@ struct Scene : SceneBase {
         const bool keys_ready = keys_fresh;
         keys_fresh = false;  // until this substep's G2P has keyed the new positions
         int64_t nk = (keys_ready ? kBinningKernelsKeysReady : kBinningKernels) + 4;
-        GMPM_TRY(launch_binning<R>(d_sc, st[c], bin, scan, d_cnt, lc.num_sms, s, keys_ready, grid_dirty));
+        GMPM_TRY(launch_bin(s, c, lc.num_sms, keys_ready));
         if (ev) GMPM_TRY(cudaEventRecord(ev[0], s));
         GMPM_TRY(launch_p2g<R>(d_sc, st[c], aux, bin, grid, d_cnt, lc, s));
         if (ev) GMPM_TRY(cudaEventRecord(ev[1], s));
@@ -599,7 +606,6 @@ struct Scene : SceneBase {
         gmpm_status r = launch_one(s, cur, ev, true, &nk);
         if (r != GMPM_OK) return r;
         commit_substeps(1);
-        grid_dirty = false;
         launches += nk - kernels_per_substep();
         return GMPM_OK;
     }
@@ -623,7 +629,6 @@ struct Scene : SceneBase {
         if (own_launches) launches += (int64_t)nsub * kernels_per_substep();  // as launched by a captured substep
         if (nsub & 1) cur = 1 - cur;
         binned = false;
-        grid_dirty = true;  // unless one_substep says otherwise
     }
     void set_sm_share(int sms) override { share_ = sms > 0 ? sms : 0; }
     int sm_share() const override { return share_; }

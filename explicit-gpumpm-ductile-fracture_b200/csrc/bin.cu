@@ -542,8 +542,12 @@ cudaError_t launch_bin_no_grid(BinDev bin, ScanScratch scan, Counters* cnt, int 
 
 template <typename R>
 cudaError_t launch_binning(const SceneDev<R>* sc, const PState<R>& st, BinDev bin, ScanScratch scan, Counters* cnt,
-                           int num_sms, cudaStream_t stream, bool keys_ready, bool clear_grid) {
-    if (clear_grid) cudaMemsetAsync(bin.grid_flag, 0, bin.key_space, stream);
+                           int num_sms, cudaStream_t stream, bool keys_ready, bool reset) {
+    if (reset) {
+        cudaMemsetAsync(bin.grid_flag, 0, bin.key_space, stream);
+        cudaMemsetAsync(bin.cell_count, 0, (size_t)bin.nb_cap * 64 * sizeof(int32_t), stream);
+        cudaMemsetAsync(scan.words, 0, (size_t)scan.count * sizeof(uint32_t), stream);
+    }
     if (!keys_ready) {
         cudaMemsetAsync(bin.page_flag, 0, bin.key_space, stream);
         k_bin_keys<R><<<bin_ctas(bin.n, kBinILP), kBinThreads, 0, stream>>>(bin.n, st.x[0], st.x[1], st.x[2], sc, bin.keys,
@@ -612,14 +616,15 @@ __device__ __forceinline__ void compact_keys_body(VB vb, uint32_t key_space, con
         raise_flag(cnt, GMPM_FLAG_TABLE_OVERFLOW);
 }
 
-// which: 1 grid flags; 2 cell counters; 3 cell counters and page flags (after
-// the page flags' last use in the binning, for the G2P that sets them).
+// which: 1 grid flags; 2 cell counters; 3 cell counters and the flags (after
+// their last use in the binning: the page flags for the G2P that sets them, the
+// grid flags for a binning of the scene by itself, which expects them zero).
 template <typename R>
 __global__ void __launch_bounds__(256) k_batch_zero(const SceneArgs<R>* __restrict__ A, const int32_t* __restrict__ start,
                                                     int ns, int which) {
     VB vb;
     const BinDev& bin = A[scene_of_block(start, ns, vb)].bin;
-    if (which == 1) zero_bytes_body(vb, bin.grid_flag, bin.key_space);
+    if (which != 2) zero_bytes_body(vb, bin.grid_flag, bin.key_space);
     if (which >= 2) zero_bytes_body(vb, bin.cell_count, (int64_t)bin.nb_cap * 64 * 4);
     if (which == 3) zero_bytes_body(vb, bin.page_flag, bin.key_space);
 }

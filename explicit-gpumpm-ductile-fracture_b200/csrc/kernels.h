@@ -54,10 +54,11 @@ struct LaunchCfg {
 // st's positions (written by the G2P that produced them), so the key pass is
 // skipped and the page flags are cleared after their last use, for the next
 // G2P to set.  Otherwise the key pass runs and the flags stay set.
-// clear_grid: a batched binning left its grid flags set.
+// Its working words (scan.words, cell_count, grid_flag) are zero between binnings, batched ones too; reset: they may not
+// be, since a launch of the last binning failed.
 template <typename R>
 cudaError_t launch_binning(const SceneDev<R>* sc, const PState<R>& st, BinDev bin, ScanScratch scan, Counters* cnt,
-                           int num_sms, cudaStream_t stream, bool keys_ready = false, bool clear_grid = false);
+                           int num_sms, cudaStream_t stream, bool keys_ready = false, bool reset = false);
 // Kernels launched by launch_binning without / with keys_ready.
 constexpr int kBinningKernels = 7;
 constexpr int kBinningKernelsKeysReady = 6;

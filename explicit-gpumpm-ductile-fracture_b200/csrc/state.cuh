@@ -59,7 +59,7 @@ struct BinDev {
     int32_t* perm;          // [n] new slot -> previous slot
     uint8_t* page_flag;     // [key_space]
     int32_t* page_rank;     // [key_space] rank of each flagged page
-    uint8_t* grid_flag;     // [key_space] zero between binnings, except after a batched one
+    uint8_t* grid_flag;     // [key_space] zero between binnings
     int32_t* grid_rank;     // [key_space]
     uint32_t* block_keys;   // [nb_cap]
     int32_t* cell_count;    // [nb_cap*64] histogram, then scatter fill pointers; zero between binnings
