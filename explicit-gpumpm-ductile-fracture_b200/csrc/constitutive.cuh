@@ -286,6 +286,10 @@ __device__ __forceinline__ void neo_hookean_fracture_from_svd(const MaterialDev<
     o.vol = V0 * det3(Fin);
 }
 
+// The least ratio of two singular values at the small strains' bound,
+// |G| <= 0.1 for G = F F^T - I: eigenvalues a and b of G with a^2 + b^2 <= 0.01 give sqrt((1 + a) / (1 + b)) >= 0.9316.
+constexpr float kSmallStrainRatio = 0.93f;
+
 // FP32 von Mises update for small strains, |F F^T - I| <= 0.1 and det F > 0
 // (Frobenius; false otherwise, and where the projected strain is larger).  The model is
 // isotropic, so every quantity is a polynomial I, G, G^2 of G = F F^T - I, with
@@ -440,17 +444,18 @@ __device__ __forceinline__ bool small_strain_update(const MaterialDev<MR>& m, fl
     o.psi = psi;
     o.vol = V0 * det3(o.F);
     o.svd_ok = true;
-    o.smin_over_smax = 0.8f;  // a lower bound: the singular values lie within sqrt(1 -+ 0.1)
+    o.smin_over_smax = kSmallStrainRatio;
     return true;
 }
 
 // The material's energy model, after one SVD of F.  kAnyModel = false
 // compiles the von Mises model alone (scenes whose materials all use it).
+// small: small strains may take the update by invariants.
 template <typename R, typename MR, bool kAnyModel = true, bool kSmallYield = true>
 __device__ __forceinline__ void constitutive_update(const MaterialDev<MR>& m, R V0, R dx, const R* Fin, R g_old,
-                                                    R alpha, R c, R psi, StressOut<R>& o) {
+                                                    R alpha, R c, R psi, StressOut<R>& o, bool small = true) {
     if constexpr (sizeof(R) == 4)
-        if ((!kAnyModel || m.energy_model == GMPM_ENERGY_VON_MISES_FRACTURE) &&
+        if (small && (!kAnyModel || m.energy_model == GMPM_ENERGY_VON_MISES_FRACTURE) &&
             small_strain_update<MR, kSmallYield>(m, V0, Fin, g_old, alpha, c, psi, o))
             return;
     R U[9], V[9], S[3];

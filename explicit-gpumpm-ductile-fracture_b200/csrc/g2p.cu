@@ -569,7 +569,9 @@ __device__ __forceinline__ void g2p_body(VB vb, const SceneDev<R>* __restrict__ 
             const R g_old = c_old * c_old * M.one_minus_theta + M.theta;
             const R alpha_in = w2.v[1], psi_in = w2.v[2];
             StressOut<R> so;
-            constitutive_update<R, R, kAnyModel, !kFallback>(M, V0, dx, Fo, g_old, alpha_in, c_new, psi_in, so);
+            // a threshold above the invariants' bound needs the singular values themselves
+            const bool small = !kFallback || ratio <= R(kSmallStrainRatio);
+            constitutive_update<R, R, kAnyModel, !kFallback>(M, V0, dx, Fo, g_old, alpha_in, c_new, psi_in, so, small);
             if (fallback && so.smin_over_smax < ratio) {
                 // FP64 SVD + return map for ill-conditioned F
                 double Fd[9];

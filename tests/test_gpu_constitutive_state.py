@@ -148,3 +148,28 @@ def test_update_matches_oracle(pkg, ctx, oracle, tmp_path, mixed, yields, trace)
     print("".join(f"\n  {k}: largest share of its bound {np.max(e / b):.3f}" for k, (e, b) in checks.items()))
     for k, (e, b) in checks.items():
         assert np.all(e <= b), (k, int(np.argmax(e / b)), float(np.max(e / b)))
+
+
+def test_fallback_threshold_above_the_small_strains(pkg, ctx, tmp_path):
+    """A threshold of 0.9 sends no small strain to FP64 (their singular values differ by less), so it changes
+    nothing; one above 1 sends every state there."""
+    G = pkg.gmpm
+    F = _states(np.random.default_rng(11), 1500, 1.0)
+    M = F.reshape(-1, 3, 3)
+    F = F[np.linalg.norm(np.transpose(M, (0, 2, 1)) @ M - np.eye(3), axis=(1, 2)) < 0.09]
+    stress = {}
+    for ratio in (1e-3, 0.9, 0.999, 1.1):
+        path = tmp_path / "state.gmpm"
+        scene, d, *_ = _load_state(pkg, ctx, path, G.PRECISION_FP32_FP64SVD, F)
+        scene.close()
+        raw = bytearray(path.read_bytes())
+        at = HEADER + G.SceneDesc.svd_fallback_ratio.offset
+        raw[at:at + 8] = np.float64(ratio).tobytes()
+        path.write_bytes(raw)
+        scene = G.Scene.load(ctx, path)
+        scene.substep(1)
+        assert scene.sync() == G.OK
+        stress[ratio] = scene.read("stress")
+    assert np.array_equal(stress[0.9], stress[1e-3])
+    assert not np.array_equal(stress[1.1], stress[1e-3])
+    assert np.array_equal(stress[0.999], stress[1.1])  # strains of 0.003 and more are below it
