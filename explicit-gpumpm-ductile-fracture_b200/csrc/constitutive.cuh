@@ -338,7 +338,8 @@ __device__ __forceinline__ bool small_strain_update(const MaterialDev<MR>& m, fl
     const float n2 = B[0] + B[1] + B[2];  // |G|^2
     if (!(n2 <= 0.01f)) return false;
     // F F^T does not tell a reflection from a rotation; the SVD path does, and its stress is then not a number
-    if (!(det3(Fin) > 0.f)) return false;
+    float J = det3(Fin);
+    if (!(J > 0.f)) return false;
     // eps = 1/2 log(I + G) = e0 I + e1 G + e2 G^2, with (p0, p1, p2) the coefficients of G^3, G^4, ...
     const float i1 = A[0] + A[1] + A[2], i2 = 0.5f * (i1 * i1 - n2), i3 = det(A);
     float e0 = 0.f, e1 = 0.5f, e2 = -0.25f;
@@ -443,10 +444,11 @@ __device__ __forceinline__ bool small_strain_update(const MaterialDev<MR>& m, fl
             o.F[3 * k + 1] = X[3] * f0 + X[1] * f1 + X[5] * f2;
             o.F[3 * k + 2] = X[4] * f0 + X[5] * f1 + X[2] * f2;
         }
+        J = det3(o.F);
     }
     o.alpha = alpha_out;
     o.psi = psi;
-    o.vol = V0 * det3(o.F);
+    o.vol = V0 * J;
     o.svd_ok = true;
     o.smin_over_smax = kSmallStrainRatio;
     return true;
