@@ -583,7 +583,9 @@ void batch_scene_ctas(int64_t n, uint32_t key_space, int nb_cap, int ng_cap, int
     ctas[BM_LINKS] = cdiv((int64_t)std::max(nb_cap, ng_cap) * 8, 256);
     ctas[BM_ZERO_CELLS] = cdiv(ncell * 4, 4096);
     ctas[BM_CELL_TILES] = (int)scan_tiles(ncell);
-    ctas[BM_CANON] = std::min(cdiv(nb_cap, kCanonWarps), sms * 8);
+    // a page for each warp of the live half of the capacity: beside many scenes, CTAs of few pages cost more than they
+    // give (64 bars: 67 us with twice as many, 44 with these)
+    ctas[BM_CANON] = std::min(cdiv(nb_cap, 2 * kCanonWarps), sms * 8);
     ctas[BM_P2G] = real_bytes == 4 ? p2g_ctas<float>(nb_cap, sms) : p2g_ctas<double>(nb_cap, sms);
     ctas[BM_GRID] = std::max(1, std::min(ng_cap / 4 + 1, sms * 8));
     const int per_sm = real_bytes == 4 ? 2 : 1;  // G2P's resident CTAs per SM
