@@ -37,7 +37,7 @@ struct PcgDev {
 
 struct GridDev {
     void* tile;        // [nb_cap][kP2GChannels][216] P2G page tiles (Real); also the solve's FP64 node tiles
-    void* nodes;       // [ng_cap][kGridChannels][64] grid results (Real)
+    void* nodes;       // [ng_cap][kGridChannels * 64] grid results (Real; grid_channel_at, common.cuh)
     double* diag;      // [8] FP64 accumulators: grid mass, grid momentum xyz, ...
     PcgDev pcg;        // implicit phase field only (null pointers otherwise)
 };

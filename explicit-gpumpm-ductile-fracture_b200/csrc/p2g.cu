@@ -3,17 +3,21 @@
 // preConditionP2G_APIC, AxP2G_APIC: P2GKernal.cu:897-1326).
 //
 // Each CTA walks its particle pages (grid-stride) in chunks of up to kP2GChunk
-// sorted slots (a whole page of 8 particles per cell).  A page's particles
+// sorted slots (a whole page of 8 particles per cell; denser pages are cut into
+// runs of cells, CellChunkIter).  A page's particles
 // share the page's 6x6x6 node window and, within a cell, the same 3x3x3
 // stencil.  Between substeps the particle planes are in the previous sorted
 // order and perm is close to the identity, so the 28 raw input planes of a
 // chunk are fetched as contiguous windows of previous slots with bulk copies
-// (one thread issues them; the tensor memory accelerator moves the data) and
-// read where they land, through the slot's place in the window.  A chunk with
-// a particle whose previous slot falls outside the window (it changed page) is
-// first gathered into sorted order in shared memory.
+// (one lane of every warp issues a few planes; the tensor memory accelerator
+// moves the data) and read where they land, through the slot's place in the
+// window.  A chunk with a particle whose previous slot falls outside the window
+// (it changed page) is first gathered into sorted order in shared memory: nearly
+// every chunk of a scene's first substep, whose previous order is the caller's,
+// and 3 to 9% of the chunks of 8.4M-particle plates 100 to 300 substeps on.
 //
-// Work split: one lane per cell and channel group.  A lane walks its cell's
+// Work split: one lane per cell and channel group (in dense pages several lanes
+// share a cell and add their sums by shuffles).  A lane walks its cell's
 // particles and keeps the cell's 27 node sums of its channels in registers, so
 // a particle costs each lane its weights once and 27 fused multiply-adds per
 // term and channel, with no shuffles and no atomics.  The groups, one per pair
@@ -34,13 +38,13 @@
 // in both modes of the scene.  The grid kernel sums the eight page tiles
 // overlapping each grid page in fixed slot order.
 //
-// Bound: neither HBM (17% of the copy rate) nor one pipe, but the chain of a
-// page's phases (copy 2,000 cycles, sweep 9,000, gather 3,000), which the two
-// CTAs of an SM overlap in part: 54% of the issue slots, FMA pipe 46%, shared
-// memory 49%.  Measured on FP32 plates: 0.718 ms at 8.4M particles and 2.73 ms
-// at 33.5M, where one lane per stencil column, all lanes on the same particle,
-// took 1.209 and 4.67 (88 warp instructions a particle against 51: every
-// particle's words were read, and its weights formed, by 27 lanes).
+// Bound: neither HBM (19% of its peak) nor one pipe, but the chain of a page's
+// phases (copy 2,000 cycles, sweep 9,000, gather 3,000), which the two CTAs of an
+// SM overlap in part: 54% of the issue slots, FMA pipe 48%, shared memory 47%.
+// Measured on FP32 plates: 0.73 ms at 8.4M particles and 2.78 ms at 33.5M, where
+// one lane per stencil column, all lanes on the same particle, took 1.209 and
+// 4.67 (88 warp instructions a particle against 52: every particle's words were
+// read, and its weights formed, by 27 lanes).
 #include <cstdint>
 
 #include "launch.cuh"
